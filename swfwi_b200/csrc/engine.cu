@@ -6,6 +6,7 @@
 #include <utility>
 #include "engine.hpp"
 #include "precond.hpp"
+#include "resident.cuh"
 
 namespace swfwi {
 
@@ -362,6 +363,24 @@ void Propagator::upload_geometry() {
       SWFWI_REQUIRE(std::adjacent_find(r.begin(), r.end()) == r.end(), "duplicate receiver positions");
     }
   }
+  row_src1_.assign(nxpad, 0);
+  row_src_.assign(nxpad, 0);
+  row_rec_.assign(nxpad, 0);
+  row_geo_.assign(nxpad, 0);
+  for (int i = 0; i < ns; i++) {
+    row_src1_[sx[i]] = 1;
+    row_src_[sx[i]]++;
+  }
+  for (int i = 0; i < ng; i++) row_geo_[gxp[i]]++;
+  rec_unused_ = false;
+  for (int s = 0; s < ns; s++) {
+    std::vector<int> h(nxpad, 0);
+    for (int i = 0; i < ngmax; i++) {
+      const int x = rx[(size_t)s * ngmax + i];
+      if (x < 0) rec_unused_ = true;
+      else row_rec_[x] = std::max(row_rec_[x], ++h[x]);
+    }
+  }
   d_src_pos_.upload(sp, st_);
   d_src_pos_p_.upload(spp, st_);
   d_src_x_.upload(sx, st_);
@@ -713,11 +732,132 @@ void Propagator::restore_snapshot(Work<T> &w, int n, int m, T *a, T *b) {
   }
 }
 
+// ---- resident time loops (resident.cuh) ----------------------------------
+bool Propagator::resident_allowed() const {
+  // the streaming kernels serve explicit launch shapes, fused loops and
+  // launches being timed
+  return stream_kernel == 6 && stream_xchunk <= 0 && !fuse && !step_timer().enabled.load(std::memory_order_relaxed);
+}
+
+// The faster one by estimate; a resident sweep has to be clearly so, since
+// the estimates are good to about 15 %.
+bool Propagator::resident_faster(const ResidentPlan &p, bool back, int n) const {
+  return p.ok && resident_us(p, arith, back) <
+                     0.87 * streamed_us(arith, back, (double)n * nxpad * nzpad, vel_stride_ != 0);
+}
+
+bool Propagator::resident_forward(Work<float> &w, int n, PointSet src, const float *vals, long long it_stride,
+                                  long long slot_stride, int i_stride, PointSet rec, int ngrec, float *dcal,
+                                  bool save_strips, const float *velrcp) {
+  if (!resident_allowed()) return false;
+  if (save_strips && (recon != SWFWI_RECON_STRIPS || strip_format != SWFWI_STRIP_F32 || illum)) return false;
+  const bool geo = rec.pos == d_geo_pos_p_.get();
+  const ResidentPlan p = plan_resident(false, n, nxpad, nzpad, bx0, save_strips, src.per_shot == 1 ? row_src1_ : row_src_,
+                                       geo ? row_geo_ : row_rec_);
+  if (!resident_faster(p, false, n)) return false;
+  if (save_strips) {   // the backward sweep reads the final pair, border zeros included
+    w.p0.zero(st_);
+    w.p1.zero(st_);
+  }
+  if (dcal && !geo && rec_unused_) SWFWI_CUDA(cudaMemsetAsync(dcal, 0, sizeof(float) * (size_t)n * nt * ngrec, st_));
+  res_halo_.resize(p.halo);
+  for (int s0 = 0; s0 < n; s0 += p.slots) {
+    ResidentArgs a{};
+    a.nx = nxpad;
+    a.nz = nzpad;
+    a.pitch = pitch;
+    a.fstride = fstride;
+    a.nt = a.steps = nt;
+    a.bx0 = bx0;
+    a.bsize = bsize;
+    a.rcp = velrcp + s0 * vel_stride_;
+    a.vel_stride = vel_stride_;
+    a.coef_x = coef_x_.get();
+    a.damp_x = damp_x_.get();
+    a.damp_z = damp_z_.get();
+    a.ramp = bx0;
+    a.p0 = w.p0.get() + kStreamCoff + s0 * fstride;
+    a.p1 = w.p1.get() + kStreamCoff + s0 * fstride;
+    a.store_state = save_strips ? 1 : 0;
+    a.src = src;
+    a.rec = rec;
+    if (src.slot_shot) a.src.slot_shot += s0;
+    if (rec.slot_shot) a.rec.slot_shot += s0;
+    a.vals = vals + s0 * slot_stride;
+    a.it_stride = it_stride;
+    a.slot_stride = slot_stride;
+    a.i_stride = i_stride;
+    a.dcal = dcal ? dcal + (long long)s0 * nt * ngrec : nullptr;
+    a.ngrec = ngrec;
+    a.strips = save_strips ? w.strips.get() + (long long)s0 * nt * bsize : nullptr;
+    a.dt = dt;
+    a.halo = res_halo_.get();
+    a.err = d_err_.get();
+    launch_resident(arith, false, p, a, std::min(p.slots, n - s0), st_);
+  }
+  return true;
+}
+
+bool Propagator::resident_backward(Work<float> &w, int n, PointSet src, const float *vals, long long it_stride,
+                                   long long slot_stride, int i_stride, PointSet rec, int ngrec, const float *vsrc,
+                                   const float *velrcp) {
+  if (!resident_allowed()) return false;
+  if (recon != SWFWI_RECON_STRIPS || strip_format != SWFWI_STRIP_F32) return false;
+  const ResidentPlan p = plan_resident(true, n, nxpad, nzpad, bx0, true, src.per_shot == 1 ? row_src1_ : row_src_,
+                                       rec.pos == d_geo_pos_p_.get() ? row_geo_ : row_rec_);
+  if (!resident_faster(p, true, n)) return false;
+  int steps = 0;   // the reference's loop images while t > 0.3
+  for (int it = nt - 1; it >= 0 && (double)(dt * (float)it) > 0.3; it--) steps++;
+  if (steps == 0) return true;
+  res_halo_.resize(p.halo);
+  for (int s0 = 0; s0 < n; s0 += p.slots) {
+    ResidentArgs a{};
+    a.nx = nxpad;
+    a.nz = nzpad;
+    a.pitch = pitch;
+    a.fstride = fstride;
+    a.nt = nt;
+    a.steps = steps;
+    a.bx0 = bx0;
+    a.bsize = bsize;
+    a.rcp = velrcp + s0 * vel_stride_;
+    a.vel_stride = vel_stride_;
+    a.coef_x = coef_x_.get();
+    a.damp_x = damp_x_.get();
+    a.damp_z = damp_z_.get();
+    a.ramp = bx0;
+    a.p0 = w.p0.get() + kStreamCoff + s0 * fstride;
+    a.p1 = w.p1.get() + kStreamCoff + s0 * fstride;
+    a.src = src;
+    a.rec = rec;
+    if (src.slot_shot) a.src.slot_shot += s0;
+    if (rec.slot_shot) a.rec.slot_shot += s0;
+    a.vals = vals + s0 * slot_stride;
+    a.it_stride = it_stride;
+    a.slot_stride = slot_stride;
+    a.i_stride = i_stride;
+    a.vsrc = vsrc + (long long)s0 * nt * ngrec;
+    a.ngrec = ngrec;
+    a.strips = w.strips.get() + (long long)s0 * nt * bsize;
+    a.image = w.image.get() + kStreamCoff + s0 * fstride;
+    a.dt = dt;
+    a.halo = res_halo_.get();
+    a.err = d_err_.get();
+    launch_resident(arith, true, p, a, std::min(p.slots, n - s0), st_);
+  }
+  return true;
+}
+
 template <typename T>
 void Propagator::run_forward(Work<T> &w, int n, PointSet src, const T *vals, long long it_stride,
                              long long slot_stride, int i_stride, PointSet rec, int ngrec, T *dcal,
                              bool save_strips, const void *velrcp) {
   ensure_work(w, n, save_strips);
+  if constexpr (sizeof(T) == 4) {
+    if (resident_forward(w, n, src, vals, it_stride, slot_stride, i_stride, rec, ngrec, dcal, save_strips,
+                         static_cast<const float *>(velrcp)))
+      return;
+  }
   T *p0 = w.p0.get() + kStreamCoff, *p1 = w.p1.get() + kStreamCoff;
   w.p0.zero(st_);
   w.p1.zero(st_);
@@ -777,6 +917,14 @@ bool Propagator::run_backward(Work<T> &w, int n, PointSet src, const T *vals, lo
                               long long slot_stride, int i_stride, PointSet rec, int ngrec,
                               const T *vsrc, const void *velrcp, const std::vector<PtLine> *src_lines,
                               const std::vector<PtLine> *rec_lines, bool sum_images) {
+  // (a batch whose images are summed step by step streams: its slots' fields
+  // are in different CTAs of a resident sweep)
+  if constexpr (sizeof(T) == 4) {
+    if ((n == 1 || !sum_images) &&
+        resident_backward(w, n, src, vals, it_stride, slot_stride, i_stride, rec, ngrec, vsrc,
+                          static_cast<const float *>(velrcp)))
+      return false;
+  }
   size_t f = (size_t)n * fstride;
   w.g0.resize(f);
   w.g1.resize(f);

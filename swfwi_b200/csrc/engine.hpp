@@ -17,6 +17,7 @@
 #include <vector>
 #include "common.hpp"
 #include "kernels.cuh"
+#include "resident.hpp"
 
 namespace swfwi {
 
@@ -206,6 +207,11 @@ class Propagator {
   std::vector<int> h_rec_count;
 
  private:
+  // points per padded row, the most of any slot: one shot's source, all
+  // sources, one shot's receivers, the common receiver line
+  std::vector<int> row_src1_, row_src_, row_rec_, row_geo_;
+  bool rec_unused_ = false;     // some shots have fewer than ngmax receivers
+  DevBuf<uint4> res_halo_;      // edge rows of the resident time loop
   cudaStream_t st_ = nullptr;   // 0 = the legacy default stream
   const float *vel_ = nullptr;
   DevBuf<float> rcp_;           // pitched 1/vt of the bound velocity
@@ -245,6 +251,16 @@ class Propagator {
                   std::vector<PtLine> &rec) const;
   bool ess_lines(int k, std::vector<PtLine> &src, std::vector<PtLine> &rec) const;
 
+  // The resident time loop (resident.cuh) of a sweep, where it applies and
+  // is the faster one; returns false when the sweep has to stream.
+  bool resident_allowed() const;
+  bool resident_faster(const ResidentPlan &p, bool back, int n) const;
+  bool resident_forward(Work<float> &w, int n, PointSet src, const float *vals, long long it_stride,
+                        long long slot_stride, int i_stride, PointSet rec, int ngrec, float *dcal, bool save_strips,
+                        const float *velrcp);
+  bool resident_backward(Work<float> &w, int n, PointSet src, const float *vals, long long it_stride,
+                         long long slot_stride, int i_stride, PointSet rec, int ngrec, const float *vsrc,
+                         const float *velrcp);
   // Forward time loop for n slots.  Source values:
   // vals + it*it_stride + slot*slot_stride + i*i_stride.
   template <typename T>

@@ -1,0 +1,189 @@
+// Launcher of the resident time loop (resident.cuh): how a batch is cut into
+// launches, slabs and row chunks.
+#include <algorithm>
+#include "common.hpp"
+#include "resident.hpp"
+#include "resident.cuh"
+
+namespace swfwi {
+
+namespace {
+
+constexpr size_t kMaxSmem = 227 * 1024;
+
+int device_sms() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    SWFWI_CUDA(cudaGetDevice(&dev));
+    SWFWI_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    return n;
+  }();
+  return sms;
+}
+
+int depth_groups(int nz) { return (nz - 6) / 4 + ((nz - 6) % 4 == 3 ? 1 : 0); }
+int row_floats(int nz) { return 4 * depth_groups(nz) + 8; }
+
+// most points of any `width` consecutive rows
+int window_max(const std::vector<int> &hist, int width) {
+  int sum = 0, most = 0;
+  for (int x = 0; x < (int)hist.size(); x++) {
+    sum += hist[x];
+    if (x >= width) sum -= hist[x - width];
+    most = std::max(most, sum);
+  }
+  return most;
+}
+
+// most strip cells in reach of any slab (backward)
+int stage_cells(int nx, int nz, int bx0, int cps) {
+  const int rows = nx - 12, nzs = std::max(nz - 6 - bx0, 0);
+  int most = 0;
+  auto overlap = [](int a0, int a1, int b0, int b1) { return std::max(std::min(a1, b1) - std::max(a0, b0), 0); };
+  for (int c = 0; c < cps; c++) {
+    const int ra = resident_detail::slab_first(rows, cps, c), rb = resident_detail::slab_first(rows, cps, c + 1) + 12;
+    most = std::max(most, 6 * overlap(ra, rb, bx0 - 6, nx - bx0 + 6) +
+                              nzs * (overlap(ra, rb, bx0 - 6, bx0) + overlap(ra, rb, nx - bx0, nx - bx0 + 6)));
+  }
+  return most;
+}
+
+// Row chunks of a slab of `rmax` rows: the count with the smallest estimate
+// of a step's issue time.  A warp task costs about 10 instructions a row to
+// fill the queue (12 rows), 62 for each u2 row (2 more than its outputs)
+// and 58 for each output row (25 more where it also images); a round of
+// `warps` tasks takes its tasks per scheduler times that, but no less than
+// one task alone at about 2.5 cycles an instruction.
+int row_chunks(bool back, int rmax, int ngroups, int warps) {
+  double best = 1e30;
+  int best_k = 1;
+  for (int k = 1; k <= std::min(rmax, kResidentChunks); k++) {
+    if ((long long)k * ngroups * ngroups >= (1 << 20)) break;
+    const int L = (rmax + k - 1) / k;
+    const int per_field = (k * ngroups + 29) / 30;
+    const double cost = 120.0 + 62.0 * (L + 2) + (back ? 70.0 : 58.0) * L + 60.0;
+    int left = per_field * (back ? 2 : 1);
+    double t = 0;
+    while (left > 0) {
+      const int a = std::min(left, warps);
+      t += cost * std::max(2.5, (double)((a + 3) / 4));
+      left -= a;
+    }
+    if (t < best) {
+      best = t;
+      best_k = k;
+    }
+  }
+  return best_k;
+}
+
+template <int ARITH, bool BACK>
+void launch_t(const ResidentArgs &a, size_t smem, cudaStream_t st) {
+  // raise the dynamic shared memory limit once (thread-safe static init)
+  static const cudaError_t attr = cudaFuncSetAttribute(fd_resident<ARITH, BACK>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  SWFWI_CUDA(attr);
+  ResidentArgs b = a;
+  void *args[] = {&b};
+  SWFWI_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fd_resident<ARITH, BACK>),
+                                         dim3(a.nslots * a.cps), dim3(kResidentThreads), args, smem, st));
+}
+
+}  // namespace
+
+ResidentPlan plan_resident(bool back, int n, int nx, int nz, int bx0, bool strips, const std::vector<int> &src_hist,
+                           const std::vector<int> &rec_hist) {
+  ResidentPlan p;
+  const int rows = nx - 12;
+  if (n <= 0 || rows < 1 || nz < 16) return p;
+  const int sms = device_sms(), zp = row_floats(nz);
+  if (6LL * depth_groups(nz) * depth_groups(nz) >= (1 << 20)) return p;   // the index divisions by multiplication
+  const int most = std::min(sms, std::max(rows / 6, 1));   // a slab's halo is its neighbours' edge rows
+  auto smem_of = [&](int cps, int &rmax, int &cs, int &cr, int &cg) {
+    rmax = (rows + cps - 1) / cps;
+    cs = window_max(src_hist, rmax + 12);
+    cr = window_max(rec_hist, rmax + 12);
+    cg = back && strips ? stage_cells(nx, nz, bx0, cps) : 0;
+    return resident_smem(back, rmax, zp, cs, cr, cg);
+  };
+  // fewest slabs whose fields fit beside their lists, from the fewest whose
+  // fields fit alone
+  const int floats_row = (back ? 6 : 3) * zp, fixed = (back ? 48 : 24) * zp;
+  const int rfit = ((int)(kMaxSmem / 4) - fixed) / floats_row;
+  if (rfit < 1) return p;
+  int cps = 0, rmax, cs, cr, cg;
+  for (int c = (rows + rfit - 1) / rfit; c <= most && !cps; c++)
+    if (smem_of(c, rmax, cs, cr, cg) <= kMaxSmem) cps = c;
+  if (!cps) return p;
+  const int slots_max = std::max(1, sms / cps);
+  const int rounds = (n + slots_max - 1) / slots_max;
+  p.slots = (n + rounds - 1) / rounds;
+  p.rounds = rounds;
+  p.cps = std::min(most, sms / p.slots);
+  p.smem = smem_of(p.cps, p.rmax, p.cap_src, p.cap_rec, p.cap_stage);
+  while (p.smem > kMaxSmem && p.cps > cps) p.smem = smem_of(--p.cps, p.rmax, p.cap_src, p.cap_rec, p.cap_stage);
+  if (p.smem > kMaxSmem) return ResidentPlan();
+  p.zp = zp;
+  p.ngroups = depth_groups(nz);
+  p.ogroups = (nz - 7) / 4;
+  // helper warps: with one, strips and records hold up the exchange; more
+  // than three take warps from the march (1 shot of 533 x 193, backward:
+  // 10.6 / 6.2 / 5.5 / 5.5 us a step with 1 / 2 / 3 / 4)
+  p.helpers = 3;
+  p.chunks = row_chunks(back, p.rmax, p.ngroups, kResidentThreads / 32 - p.helpers);
+  if (resident_halo(p.slots, p.cps, 2, p.ogroups) >= (1u << 31)) return ResidentPlan();
+  p.halo = resident_halo(p.slots, p.cps, back ? 2 : 1, p.ogroups);
+  p.ok = true;
+  return p;
+}
+
+// Estimated microseconds a step (B200, fits to timed sweeps of 1..96 shots of
+// 272 x 142, 533 x 193 and 993 x 343 padded points; within about 15 %).  A
+// resident round costs its latency (points, exchange, barriers) plus its
+// largest slab's march; a streamed step its launches plus its points.
+// Measured forward / backward, FAST: 1 shot of 533 x 193 3.0 / 5.5 resident
+// against 9.0 / 18.9 streamed; 20 shots 6.5 / 18.6 against 13.0 / 31.5; 96
+// shots 28.8 / 114 against 36.1 / 108; 1 shot of 993 x 343 3.8 / 8.0 against
+// 9.2 / 19.1; 10 shots 12.2 / 46 against 15.5 / 34; 96 shots 113 / 599
+// against 87 / 227.
+double resident_us(const ResidentPlan &p, int arith, bool back) {
+  const double x = (double)p.rmax * p.ngroups;
+  const bool ref = arith == ARITH_REF;
+  const double round = back ? (ref ? 3.5 + 0.0066 * x : 2.9 + 0.0028 * x) + 0.045 * p.ogroups
+                            : (ref ? 3.9 + 0.0027 * x : 2.7 + 0.00113 * x);
+  return p.rounds * round;
+}
+double streamed_us(int arith, bool back, double points, bool own_velocity) {
+  const double m = points * 1e-6;
+  if (arith == ARITH_REF) return back ? 30 + 10 * m : 14 + 3.9 * m;
+  return back ? 17.5 + 6.6 * m : 8.3 + (own_velocity ? 4.9 : 2.4) * m;
+}
+
+void launch_resident(int arith, bool back, const ResidentPlan &p, ResidentArgs a, int nslots, cudaStream_t st) {
+  a.nslots = nslots;
+  a.cps = p.cps;
+  a.rmax = p.rmax;
+  a.zp = p.zp;
+  a.ngroups = p.ngroups;
+  a.ogroups = p.ogroups;
+  a.gmagic = (1u << 20) / (unsigned)p.ngroups + 1;
+  a.omagic = (1u << 20) / (unsigned)p.ogroups + 1;
+  const int nzs = std::max(a.nz - 6 - a.bx0, 1);
+  a.nzs_magic = (unsigned)((1ull << 32) / nzs + 1);
+  a.chunks = p.chunks;
+  a.helpers = p.helpers;
+  a.cap_src = p.cap_src;
+  a.cap_rec = p.cap_rec;
+  a.cap_stage = p.cap_stage;
+  SWFWI_CUDA(cudaMemsetAsync(a.halo, 0, sizeof(uint4) * resident_halo(nslots, p.cps, back ? 2 : 1, p.ogroups), st));
+  if (arith == ARITH_REF) {
+    if (back) launch_t<ARITH_REF, true>(a, p.smem, st);
+    else launch_t<ARITH_REF, false>(a, p.smem, st);
+  } else {
+    if (back) launch_t<ARITH_FAST, true>(a, p.smem, st);
+    else launch_t<ARITH_FAST, false>(a, p.smem, st);
+  }
+  note_launch();
+}
+
+}  // namespace swfwi
