@@ -331,6 +331,46 @@ __global__ void k_prtm_born_transpose(float *cn, float *bh, const float *ah, con
 constexpr size_t kBatchBudget = size_t(24) << 30;
 
 }  // namespace
+}  // namespace swfwi
+
+#include "lsrtm_resident.cuh"
+
+namespace swfwi {
+namespace {
+
+// How a resident sweep of k shots is cut (lsrtm_resident.cuh).
+struct PrtmPlan {
+  bool ok = false;
+  int slots = 0, cps = 0, rmax = 0, zp = 0, ngroups = 0, ogroups = 0, chunks = 0, cap_rec = 0, cap_ring = 0;
+  size_t smem = 0, halo = 0;
+};
+constexpr int kPrtmHelpers = 3;   // warps for records, rings and data beside the march (1 shot, migration: 6.6 / 4.7 / 4.3 us a step with 1 / 2 / 3)
+constexpr size_t kPrtmMaxSmem = 227 * 1024;
+
+template <int ARITH, int MODE>
+void prtm_resident_launch(const PrtmResident &a, size_t smem, cudaStream_t st) {
+  // raise the dynamic shared memory limit once (thread-safe static init)
+  static const cudaError_t attr = cudaFuncSetAttribute(k_prtm_resident<ARITH, MODE>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrtmMaxSmem);
+  SWFWI_CUDA(attr);
+  PrtmResident b = a;
+  void *args[] = {&b};
+  SWFWI_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_prtm_resident<ARITH, MODE>),
+                                         dim3(a.nslots * a.cps), dim3(kPrtmThreads), args, smem, st));
+  note_launch();
+}
+
+template <int ARITH>
+void prtm_resident_mode(int mode, const PrtmResident &a, size_t smem, cudaStream_t st) {
+  switch (mode) {
+    case PRTM_BORN: prtm_resident_launch<ARITH, PRTM_BORN>(a, smem, st); break;
+    case PRTM_SOURCE: prtm_resident_launch<ARITH, PRTM_SOURCE>(a, smem, st); break;
+    case PRTM_MIGRATE: prtm_resident_launch<ARITH, PRTM_MIGRATE>(a, smem, st); break;
+    default: prtm_resident_launch<ARITH, PRTM_TRANSPOSE>(a, smem, st); break;
+  }
+}
+
+}  // namespace
 
 // The operator's state (prtm2d_init's file-scope variables, per object).
 class Prtm {
@@ -401,11 +441,30 @@ class Prtm {
     }
     ring_.resize((size_t)kmax_ * nt * 4 * (nx + nz));
     if (kmax_ > 1) img_.resize((size_t)kmax_ * nx * nz);
+    // for resident sweeps: the most receivers of any shot on each padded row
+    row_rec_.assign(nxpad_, 0);
+    for (int is = 0; is < ns; is++) {
+      std::vector<int> h(nxpad_, 0);
+      for (int ig = 0; ig < ng; ig++) {
+        const int x = rpos[(size_t)is * ng + ig] / nzpad_;
+        row_rec_[x] = std::max(row_rec_[x], ++h[x]);
+      }
+    }
+    geo_serial_ = ng > 1 && jgx == 0 && jgz == 0;
+    err_.resize(1);
+    err_.zero(st);
+    SWFWI_CUDA(cudaHostAlloc(&h_err_, sizeof(int), cudaHostAllocDefault));
+    *h_err_ = 0;
+    int dev = 0;
+    SWFWI_CUDA(cudaGetDevice(&dev));
+    SWFWI_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
+    for (int m = 0; m < 4; m++) plan_[m] = plan_resident_sweep(m);
     geo_ = PrtmGeo{nx, nz, nb, nxpad_, nzpad_, nt, ng, (long long)fsz, spos_.get(), rpos_.get(), sponge_.get(),
                    ng > 1 && jgx == 0 && jgz == 0 ? 1 : 0};
   }
 
   ~Prtm() {
+    if (h_err_) cudaFreeHost(h_err_);
     for (Graph &g : graphs_)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     if (cap_) cudaStreamDestroy(cap_);
@@ -438,7 +497,13 @@ class Prtm {
       }
       for (int s0 = 0; s0 < ns_; s0 += kmax_) run(adj, mod, dat, s0, std::min(kmax_, ns_ - s0), s);
     };
-    if (!use_graphs_) {
+    if (*h_err_) {   // as far as earlier calls are known to have finished
+      *h_err_ = 0;
+      err_.zero(st);
+      throw Error(SWFWI_ERR_TIMEOUT, "a resident sweep's bounded wait on its neighbours gave up");
+    }
+    // resident sweeps are a launch or two each: nothing for a graph to gain
+    if (!use_graphs_ || resident(adj)) {
       body(st);
       SWFWI_CUDA(cudaGetLastError());
       return;
@@ -493,6 +558,145 @@ class Prtm {
   };
   static constexpr size_t kGraphs = 4;
 
+  // ---- resident sweeps ----
+  PrtmPlan plan_resident_sweep(int mode) const {
+    PrtmPlan p;
+    // injection at one shared cell has an order; a one-step sweep exchanges
+    // nothing, so nothing would order its state's loads and stores
+    if (geo_serial_ || nt_ < 2) return p;
+    const int rows = nxpad_ - 4;
+    p.ngroups = (nzpad_ + 3) / 4;
+    p.ogroups = (nzpad_ - 3) / 4 + 1;
+    p.zp = 4 * p.ngroups;
+    if (nzpad_ < 8 || rows < 1 || p.ngroups >= 1024) return p;
+    const int most = std::min(sms_, std::max(rows / 2, 1));   // a slab's halo is its neighbours' edge rows
+    auto need = [&](int cps) {
+      p.rmax = (rows + cps - 1) / cps;
+      int sum = 0;
+      p.cap_rec = 0;
+      for (int x = 0; x < nxpad_ && mode != PRTM_SOURCE; x++) {
+        sum += row_rec_[x] - (x >= p.rmax + 4 ? row_rec_[x - p.rmax - 4] : 0);
+        p.cap_rec = std::max(p.cap_rec, sum);
+      }
+      const bool prefetch = mode == PRTM_MIGRATE || mode == PRTM_TRANSPOSE;
+      p.cap_ring = prefetch ? 4 * (p.rmax + 4) + std::min(4, p.rmax + 4) * nz_ : 0;
+      p.smem = 4 * (size_t)PrtmLayout(mode, p.rmax, p.zp, p.cap_rec, p.cap_ring).total;
+    };
+    int cps = 1;
+    for (need(cps); p.smem > kPrtmMaxSmem && cps < most;) need(++cps);
+    if (p.smem > kPrtmMaxSmem) return p;
+    const int fit = std::max(1, sms_ / cps), rounds = (kmax_ + fit - 1) / fit;
+    p.slots = (kmax_ + rounds - 1) / rounds;
+    p.cps = std::min(most, sms_ / p.slots);
+    need(p.cps);
+    p.halo = (size_t)p.slots * p.cps * (mode == PRTM_SOURCE ? 1 : 2) * 4 * 4 * p.ogroups;
+    // row chunks: about 170 instructions an output row of both pairs, 14 a
+    // row to fill the queue; a round of warps as in the propagator's sweeps
+    const int warps = kPrtmThreads / 32 - kPrtmHelpers;
+    double best = 1e30;
+    for (int k = 1; k <= std::min(p.rmax, kPrtmChunks) && (long long)k * p.ngroups * p.ngroups < (1 << 20); k++) {
+      const int L = (p.rmax + k - 1) / k;
+      double t = 0;
+      for (int left = (k * p.ngroups + 29) / 30; left > 0; left -= warps)
+        t += (120.0 + 170.0 * L) * std::max(2.5, (double)((std::min(left, warps) + 3) / 4));
+      if (t < best) {
+        best = t;
+        p.chunks = k;
+      }
+    }
+    p.ok = p.chunks > 0;
+    return p;
+  }
+  bool resident(bool adj) const {
+    if (!adj) return plan_[PRTM_BORN].ok;
+    return plan_[PRTM_SOURCE].ok && plan_[adj_mode_ == SWFWI_PRTM_ADJ_EXACT ? PRTM_TRANSPOSE : PRTM_MIGRATE].ok;
+  }
+  // one sweep over the k shots from s0 (the batch's first), images (or the
+  // model of k == 1) in img
+  void resident_sweep(int mode, float *mod, float *dat, float *img, long long img_stride, float *G0, float *G1, int s0,
+                      int k, cudaStream_t st) {
+    const PrtmPlan &p = plan_[mode];
+    halo_.resize(p.halo);
+    for (int c = 0; c < k; c += p.slots) {
+      PrtmResident a{};
+      a.g = geo_;
+      a.g.spos = spos_.get() + s0 + c;
+      a.g.rpos = rpos_.get() + (size_t)(s0 + c) * ng_;
+      a.c = c_;
+      a.nslots = std::min(p.slots, k - c);
+      a.cps = p.cps;
+      a.rmax = p.rmax;
+      a.zp = p.zp;
+      a.ngroups = p.ngroups;
+      a.ogroups = p.ogroups;
+      a.chunks = p.chunks;
+      a.helpers = kPrtmHelpers;
+      a.gmagic = (1u << 20) / (unsigned)p.ngroups + 1;
+      a.nz_magic = (unsigned)((1ull << 32) / nz_ + 1);
+      a.cap_rec = p.cap_rec;
+      a.cap_ring = p.cap_ring;
+      a.vv = vv_.get();
+      a.mod = mod;
+      a.wl = wlt_.get();
+      a.s0 = sp0_.get() + (long long)c * fsz();
+      a.s1 = sp1_.get() + (long long)c * fsz();
+      a.g0 = G0 + (long long)c * fsz();
+      a.g1 = G1 + (long long)c * fsz();
+      a.keep_g = arith_ == ARITH_REF ? 1 : 0;
+      a.dat = dat + (long long)c * nt_ * ng_;
+      a.ring_stride = (long long)nt_ * 4 * (nx_ + nz_);
+      a.ring = ring_.get() + c * a.ring_stride;
+      a.img = img ? img + c * img_stride : nullptr;
+      a.img_stride = img_stride;
+      a.halo = halo_.get();
+      a.err = err_.get();
+      SWFWI_CUDA(cudaMemsetAsync(halo_.get(), 0, sizeof(uint4) * p.halo, st));
+      if (arith_ == ARITH_REF) prtm_resident_mode<ARITH_REF>(mode, a, p.smem, st);
+      else prtm_resident_mode<ARITH_FAST>(mode, a, p.smem, st);
+    }
+  }
+  void run_resident(bool adj, float *mod, float *dat, int s0, int k, cudaStream_t st) {
+    const long long nm = (long long)nx_ * nz_;
+    const size_t fbytes = sizeof(float) * (size_t)k * fsz();
+    float *G0 = gp0_.get(), *G1 = gp1_.get();
+    if (g_swapped_) std::swap(G0, G1);
+    g_swapped_ = false;   // the sweeps write the pair in place
+    if (G0 != gp0_.get()) {   // REF: continue from the pair in its own order
+      SWFWI_CUDA(cudaMemcpyAsync(gp2_.get(), gp0_.get(), fbytes, cudaMemcpyDeviceToDevice, st));
+      SWFWI_CUDA(cudaMemcpyAsync(gp0_.get(), gp1_.get(), fbytes, cudaMemcpyDeviceToDevice, st));
+      SWFWI_CUDA(cudaMemcpyAsync(gp1_.get(), gp2_.get(), fbytes, cudaMemcpyDeviceToDevice, st));
+      G0 = gp0_.get();
+      G1 = gp1_.get();
+    }
+    float *d = dat + (long long)s0 * nt_ * ng_;
+    if (!adj) {
+      resident_sweep(PRTM_BORN, mod, d, nullptr, 0, G0, G1, s0, k, st);
+    } else {
+      const bool exact = adj_mode_ == SWFWI_PRTM_ADJ_EXACT;
+      // the sweeps write the cells they update; the border cells stay zero
+      // from the fields' creation on
+      resident_sweep(PRTM_SOURCE, mod, d, nullptr, 0, G0, G1, s0, k, st);
+      float *img = mod;
+      long long img_stride = 0;
+      if (k > 1) {
+        SWFWI_CUDA(cudaMemsetAsync(img_.get(), 0, sizeof(float) * (size_t)k * nm, st));
+        img = img_.get();
+        img_stride = nm;
+      }
+      resident_sweep(exact ? PRTM_TRANSPOSE : PRTM_MIGRATE, mod, d, img, img_stride, G0, G1, s0, k, st);
+      if (k > 1) {
+        const long long blocks = std::min<long long>((nm + 255) / 256, 148 * 16);
+        k_prtm_sum_images<<<(unsigned)blocks, 256, 0, st>>>(mod, img_.get(), nm, k);
+        note_launch();
+      }
+      if (exact) {   // as after the launched loops: no order a later REF Born could continue from
+        SWFWI_CUDA(cudaMemsetAsync(G0, 0, fbytes, st));
+        SWFWI_CUDA(cudaMemsetAsync(G1, 0, fbytes, st));
+      }
+    }
+    SWFWI_CUDA(cudaMemcpyAsync(h_err_, err_.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
+  }
+
   int pidx(int x, int z) const { return (x + nb_) * nzpad_ + z + nb_; }
   long long fsz() const { return (long long)nxpad_ * nzpad_; }
   int rec_cols(int zthreads) const { return (ng_ + zthreads - 1) / zthreads; }
@@ -542,6 +746,10 @@ class Prtm {
   // in one or two (k_prtm_aux), the reference's operations regrouped where
   // they touch disjoint cells and so commute.
   void run(bool adj, float *mod, float *dat, int s0, int k, cudaStream_t st) {
+    if (resident(adj)) {
+      run_resident(adj, mod, dat, s0, k, st);
+      return;
+    }
     const long long nm = (long long)nx_ * nz_;
     const size_t fbytes = sizeof(float) * (size_t)k * fsz();
     // the batch's positions
@@ -682,7 +890,13 @@ class Prtm {
 
   int arith_, nz_, nx_, nb_, nt_, ns_, ng_, nzpad_ = 0, nxpad_ = 0;
   int kmax_ = 1, adj_mode_ = SWFWI_PRTM_ADJ_REFERENCE;
-  bool g_swapped_ = false, use_graphs_ = true;
+  bool g_swapped_ = false, use_graphs_ = true, geo_serial_ = false;
+  int sms_ = 148;
+  PrtmPlan plan_[4];               // by PrtmSweep
+  std::vector<int> row_rec_;
+  DevBuf<uint4> halo_;
+  DevBuf<int> err_;
+  int *h_err_ = nullptr;
   PrtmCoef c_{};
   PrtmGeo geo_{};
   DevBuf<float> vv_, wlt_, sponge_, sp0_, sp1_, gp0_, gp1_, gp2_, ring_, img_;

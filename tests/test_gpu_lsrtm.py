@@ -204,3 +204,33 @@ def test_graph_replay_counts_its_kernels(cuda):
         counts.append(S.stats_read()["kernel_launches"])
         op.close()
     assert counts[0] == counts[1] and counts[0] > 0, counts
+
+
+@pytest.mark.parametrize("arith", [0, 1])
+@pytest.mark.parametrize("nx,nz,nb,ns,ng", [(3, 4, 2, 1, 2), (21, 30, 3, 2, 21), (40, 33, 10, 3, 40), (61, 42, 11, 5, 30),
+                                            (300, 25, 12, 1, 300), (90, 150, 10, 70, 45)])
+def test_resident_sweeps_match_fp64(cuda, arith, nx, nz, nb, ns, ng):
+    """The operator with its fields held on chip, at slabs of 2 rows and up,
+    depths that are and are not multiples of the 4-depth groups and batches
+    of several launches: modelling, and the exact adjoint on its data."""
+    import swfwi_b200 as S
+    torch = cuda
+    rng = np.random.default_rng(nx)
+    vel = (1800.0 + 15.0 * np.arange(nz)[None, :] + 40.0 * rng.random((nx, nz))).astype(np.float32)
+    mod = rng.standard_normal((nx, nz)).astype(np.float32)
+    if arith == S.ARITH_REF:
+        ns = 1      # its shots continue from one another's fields; the restatement's start from zero
+    a = dict(dz=10.0, dx=10.0, dt=0.001, amp=1.0, fm=25.0, nb=nb, nt=121, ns=ns, ng=ng, sxbeg=0, szbeg=1,
+             jsx=(nx - 1) // ns, jsz=0, gxbeg=0, gzbeg=2, jgx=max(1, (nx - 1) // max(ng - 1, 1)), jgz=0)
+    o = PrtmF64(vel, **a)
+    op = S.Prtm2d(t(torch, vel), arith=arith, **a)
+    d = torch.zeros((ns, ng, a["nt"]), device="cuda")
+    op.lop(False, False, t(torch, mod), d)
+    want = o.born(mod)
+    assert rel_l2(d.cpu().numpy(), want) < TOL_FAST
+    if nb >= 10:    # thinner sponges drift in the FP32 reconstruction (above)
+        op.set_adjoint(S.PRTM_ADJ_EXACT)
+        m = torch.zeros((nx, nz), device="cuda")
+        op.lop(True, False, m, t(torch, want.astype(np.float32)))
+        assert rel_l2(m.cpu().numpy(), o.born_transpose(want.astype(np.float32))) < EXACT_TOL["line"]
+    op.close()
