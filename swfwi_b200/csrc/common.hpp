@@ -49,6 +49,33 @@ int guarded(F &&f) {
   }
 }
 
+// cudaMalloc; if the device is full, once more without this context's kept
+// scratch.
+void *device_alloc(size_t bytes);
+// Frees the scratch kept for the current context; false: there was none.
+bool release_kept_scratch();
+
+// Device scratch of a call that returns synchronised: taken from the buffer
+// kept for the context if it is large enough and free, else allocated.  Once
+// the work that uses it has ended the call says so by idle(), and the buffer
+// may be kept; without that (an exception) it is freed, which waits.
+class Scratch {
+ public:
+  explicit Scratch(size_t bytes);
+  ~Scratch();
+  Scratch(const Scratch &) = delete;
+  Scratch &operator=(const Scratch &) = delete;
+  void *get() const { return p_; }
+  void idle() { idle_ = true; }
+
+ private:
+  int dev_ = 0;
+  unsigned long long ctx_ = 0;
+  void *p_ = nullptr;
+  size_t bytes_ = 0;
+  bool idle_ = false;
+};
+
 // Owning device allocation (cudaMalloc / cudaFree).
 template <typename T>
 class DevBuf {
@@ -75,7 +102,7 @@ class DevBuf {
   void resize(size_t n) {
     if (n > cap_) {
       release();
-      SWFWI_CUDA(cudaMalloc(&p_, n * sizeof(T)));
+      p_ = static_cast<T *>(device_alloc(n * sizeof(T)));
       cap_ = n;
     }
     n_ = n;

@@ -12,16 +12,17 @@
 // and s_i^2, V the eigenpairs of X1.  The three N x N cross products are
 // the only work over the data (O(rows N^2)); one fused pass forms them row
 // by row (row means, perturbation, band and residual never reach HBM), a
-// fixed-order reduction sums the per-CTA partials, and one CTA solves the
-// N x N eigen problem (parallel-ordered two-sided Jacobi in FP64 shared
-// memory), sorts it, applies clipPosition and forms t4, which stays in
-// device memory for the member update.
+// fixed-order reduction sums the per-CTA partials, one CTA solves the N x N
+// eigen problem (parallel-ordered two-sided Jacobi in FP64 shared memory),
+// sorts it and applies clipPosition, and a few small kernels form V and t4,
+// which stays in device memory for the member update.
 //
 // analyze (enkfanalyze.cpp:57-111) then moves each member by
 // A' t4 (A' = members - their float mean), in physical velocity.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <vector>
 #include "common.hpp"
 #include "kernels.cuh"
@@ -30,7 +31,6 @@ namespace swfwi {
 namespace {
 
 constexpr int kMaxMembers = 64;   // members per analysis (one 64 x 64 tile)
-constexpr int kRowsPerChunk = 16;
 constexpr int kThreads = 256;
 
 // ---- counter-based normal draws (Philox4x32-10 of Salmon et al. 2011,
@@ -94,133 +94,235 @@ __global__ void k_value_at(double *sigma, const unsigned long long *best, const 
   *sigma = fabs((double)hona[i0 * rows + r] - s / n) * (double)sigfac;
 }
 
-// ---- the three cross products, one pass over the rows.  A CTA takes 16
-// rows at a time: it stages the members' HA and perturbation of those rows
-// in shared memory, forms the row means in member order (as initGamma
-// sums), then HA', band and D - HA; each thread accumulates a 4 x 4 tile of
-// X1, X2 and X3 over the rows.  partials[cta][3][64][64].
+// D += A B on the FP64 tensor cores: A 8 x 4 (lane: row lane / 4, column
+// lane % 4), B 4 x 8 (row lane % 4, column lane / 4), D row lane / 4,
+// columns 2 * (lane % 4) and the next.
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// ---- the three cross products, one pass over the rows, a CTA per SM and 32
+// rows at a time.  A warp takes 8 rows x 16 members (a lane 4 members of a
+// row): it reads HA, draws the perturbation, sums both by row, and once the
+// four warps of a row have their sums writes HA', band and D - HA to shared
+// memory, [member][row] with a stride that serves the products' fragments
+// (an A and a B fragment of the same operand are the same 8 x 4 values)
+// without bank conflicts.  The products run on the FP64 tensor cores, an
+// 8 x 32 strip of X1, X2 and X3 a warp, while half of the warps draw the
+// next rows.  Both use the FP64 pipe, which bounds it: 61 % busy, 44 with
+// products and 17 with draws.  461000 rows of 64 members: 0.71 ms; 1.92 with
+// 4 x 4 tiles of plain FP64 a thread, row sums by 16 threads of 256 and
+// everything in turn.  partials[cta][3][64][64].
+constexpr int kCrossThreads = 512;
+constexpr int kRows = 32;         // rows of a chunk
+constexpr int kLdr = kRows + 4;   // 4 mod 16: an 8 x 4 fragment covers the banks once
+
+__host__ __device__ constexpr size_t cross_smem_bytes() {
+  return sizeof(double) * (3 * kMaxMembers * kLdr + 2 * 4 * kRows);
+}
+
 template <bool DRAW>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kCrossThreads, 1)
 k_cross(double *partials, const float *hona, const float *dobs, const double *z, long long rows, int n,
         const double *sigma_dev, unsigned long long seed) {
+  extern __shared__ __align__(16) double cross_sm[];
+  double *sh = cross_sm;                        // HA'   [64][kLdr]
+  double *sp = sh + kMaxMembers * kLdr;         // band
+  double *sr = sp + kMaxMembers * kLdr;         // D - HA
+  double *sums = sr + kMaxMembers * kLdr;       // [2][member set][row]
   const double sigma = *sigma_dev;
-  __shared__ double sh[kRowsPerChunk][kMaxMembers];   // HA, then HA'
-  __shared__ double sp[kRowsPerChunk][kMaxMembers];   // perturbation, then band
-  __shared__ double st[kRowsPerChunk][kMaxMembers];   // D - HA
-  __shared__ double mh[kRowsPerChunk], mp[kRowsPerChunk];
-  const int t = threadIdx.x, ta = t >> 4, tb = t & 15, lr = t & 15;
-  double a1[4][4] = {}, a2[4][4] = {}, a3[4][4] = {};
-  for (long long r0 = (long long)blockIdx.x * kRowsPerChunk; r0 < rows;
-       r0 += (long long)gridDim.x * kRowsPerChunk) {
-    const long long r = r0 + lr;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // producer: row lrow of the chunk, members 16 * set + 4 * q + lane / 8
+  const int set = warp >> 2, lrow = (warp & 3) * 8 + (lane & 7), m0 = 16 * set + (lane >> 3);
+  // products: rows of tile ti, columns of tiles tj .. tj+3
+  const int ti = warp >> 1, tj = (warp & 1) * 4, tiles = (n + 7) / 8;
+  const int frag = (lane >> 2) * kLdr + (lane & 3);
+  double a1[4][2] = {}, a2[4][2] = {}, a3[4][2] = {};
+  double h[4], p[4], d = 0.0;
+
+  auto draw = [&](long long r0) {
+    const long long r = r0 + lrow;
     const bool rok = r < rows;
+    double s = 0.0, u = 0.0;
+    d = rok ? (double)dobs[r] : 0.0;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      const int i = (t >> 4) + 16 * q;
-      double h = 0.0, p = 0.0;
+      const int i = m0 + 4 * q;
+      h[q] = p[q] = 0.0;
       if (rok && i < n) {
-        h = (double)hona[i * rows + r];
-        p = sigma * (DRAW ? normal_draw(seed, (unsigned long long)(i * rows + r)) : z[i * rows + r]);
+        h[q] = (double)hona[i * rows + r];
+        p[q] = sigma * (DRAW ? normal_draw(seed, (unsigned long long)(i * rows + r)) : z[i * rows + r]);
       }
-      sh[lr][i] = h;
-      sp[lr][i] = p;
+      s += h[q];
+      u += p[q];
     }
-    __syncthreads();
-    if (t < kRowsPerChunk) {
-      double a = 0.0, b = 0.0;
-      for (int i = 0; i < n; i++) {
-        a += sh[t][i];
-        b += sp[t][i];
-      }
-      mh[t] = a / n;
-      mp[t] = b / n;
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+      u += __shfl_xor_sync(0xffffffffu, u, o);
     }
-    __syncthreads();
-    const double d = rok ? (double)dobs[r] : 0.0;
+    if (lane < 8) {
+      sums[set * kRows + lrow] = s;
+      sums[(4 + set) * kRows + lrow] = u;
+    }
+  };
+  auto finish = [&](long long r0) {
+    const bool rok = r0 + lrow < rows;
+    double s = 0.0, u = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      s += sums[k * kRows + lrow];
+      u += sums[(4 + k) * kRows + lrow];
+    }
+    const double mh = s / n, mp = u / n;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      const int i = (t >> 4) + 16 * q;
-      double hap = 0.0, band = 0.0, res = 0.0;
-      if (rok && i < n) {
-        const double h = sh[lr][i], p = sp[lr][i];
-        hap = h - mh[lr];
-        band = hap + (p - mp[lr]);
-        res = (d + p) - h;
-      }
-      sh[lr][i] = hap;
-      sp[lr][i] = band;
-      st[lr][i] = res;
+      const int i = m0 + 4 * q;
+      const bool ok = rok && i < n;
+      const double hap = h[q] - mh;
+      sh[i * kLdr + lrow] = ok ? hap : 0.0;
+      sp[i * kLdr + lrow] = ok ? hap + (p[q] - mp) : 0.0;
+      sr[i * kLdr + lrow] = ok ? (d + p[q]) - h[q] : 0.0;
     }
-    __syncthreads();
-#pragma unroll 4
-    for (int rr = 0; rr < kRowsPerChunk; rr++) {
-      double ga[4], ha[4], gb[4], tb4[4];
+  };
+  auto products = [&] {
+    if (ti >= tiles || tj >= tiles) return;
+#pragma unroll 2
+    for (int k = 0; k < kRows; k += 4) {
+      const double gb = sp[ti * 8 * kLdr + frag + k], gh = sh[ti * 8 * kLdr + frag + k];
 #pragma unroll
-      for (int x = 0; x < 4; x++) {
-        ga[x] = sp[rr][4 * ta + x];
-        ha[x] = sh[rr][4 * ta + x];
-        gb[x] = sp[rr][4 * tb + x];
-        tb4[x] = st[rr][4 * tb + x];
+      for (int j = 0; j < 4; j++) {
+        const int o = (tj + j) * 8 * kLdr + frag + k;   // members past n are zeros
+        const double b = sp[o], r = sr[o];
+        mma_f64(a1[j], gb, b);
+        mma_f64(a2[j], gh, b);
+        mma_f64(a3[j], gb, r);
       }
-#pragma unroll
-      for (int x = 0; x < 4; x++)
-#pragma unroll
-        for (int y = 0; y < 4; y++) {
-          a1[x][y] = fma(ga[x], gb[y], a1[x][y]);
-          a2[x][y] = fma(ha[x], gb[y], a2[x][y]);
-          a3[x][y] = fma(ga[x], tb4[y], a3[x][y]);
-        }
     }
-    __syncthreads();
+  };
+
+  const long long step = (long long)gridDim.x * kRows;
+  long long r0 = (long long)blockIdx.x * kRows;
+  draw(r0);
+  __syncthreads();
+  finish(r0);
+  for (; r0 < rows; r0 += step) {
+    __syncthreads();   // this chunk is in shared memory
+    if (warp & 4) {
+      products();
+      draw(r0 + step);
+    } else {
+      draw(r0 + step);
+      products();
+    }
+    __syncthreads();   // its products and the next one's sums are done
+    finish(r0 + step);
   }
   double *out = partials + (long long)blockIdx.x * 3 * kMaxMembers * kMaxMembers;
 #pragma unroll
-  for (int x = 0; x < 4; x++)
+  for (int j = 0; j < 4; j++) {
+    const int e = (ti * 8 + (lane >> 2)) * kMaxMembers + (tj + j) * 8 + 2 * (lane & 3);
 #pragma unroll
-    for (int y = 0; y < 4; y++) {
-      const int e = (4 * ta + x) * kMaxMembers + 4 * tb + y;
-      out[e] = a1[x][y];
-      out[kMaxMembers * kMaxMembers + e] = a2[x][y];
-      out[2 * kMaxMembers * kMaxMembers + e] = a3[x][y];
+    for (int c = 0; c < 2; c++) {
+      out[e + c] = a1[j][c];
+      out[kMaxMembers * kMaxMembers + e + c] = a2[j][c];
+      out[2 * kMaxMembers * kMaxMembers + e + c] = a3[j][c];
     }
+  }
 }
 
 // Sum of the per-CTA partials in CTA order (deterministic).
-__global__ void k_sum_partials(double *x, const double *partials, int nparts) {
+__global__ void __launch_bounds__(64) k_sum_partials(double *x, const double *partials, int nparts) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int m = 3 * kMaxMembers * kMaxMembers;
   if (e >= m) return;
   double s = 0.0;
+#pragma unroll 8
   for (int b = 0; b < nparts; b++) s += partials[(long long)b * m + e];
   x[e] = s;
 }
 
-// ---- analyze's update, one thread per model point: the members' float
-// mean (createAMean, enkfanalyze.cpp:568-580), A' in double, A' t4, and
-// v <- velTrans(velRecover(v) + (A' t4)_i) (enkfanalyze.cpp:72-108).
+// ---- analyze's update: the members' float mean (createAMean,
+// enkfanalyze.cpp:568-580), A' in double, A' t4, and
+// v <- velTrans(velRecover(v) + (A' t4)_i) (enkfanalyze.cpp:72-108).  A CTA
+// takes 128 model points: their values of every member stay in shared memory
+// (one read and one write of HBM), the mean is summed there in member order,
+// and A' t4 runs on the FP64 tensor cores, 16 points x all members a warp.
+// 64 members of 129519 points: 87 us; 318 with a thread per point, its 64
+// sums of 64 terms re-read from L1 and spilled.
+constexpr int kTile = 128;          // points of a CTA
+constexpr int kLdp = kTile + 8;     // floats a member row: 8 mod 32
+constexpr int kLdg = kMaxMembers + 4;   // doubles a column of t4: 4 mod 16
+
+__host__ __device__ constexpr size_t update_smem_bytes() {
+  return sizeof(double) * kMaxMembers * kLdg + sizeof(float) * (kMaxMembers * kLdp + kTile);
+}
+
 __device__ __forceinline__ void update_members(float *vels, long long model, int n, const double *t4, float dx,
                                                float dt) {
-  __shared__ double g[kMaxMembers * kMaxMembers];   // t4 column-major: row j, col i at i*n + j
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) g[e] = t4[e];
-  __syncthreads();
+  extern __shared__ __align__(16) double update_sm[];
+  double *g = update_sm;                                      // t4, column i at i * kLdg, zeros past n
+  float *sv = reinterpret_cast<float *>(g + kMaxMembers * kLdg);   // [64][kLdp]
+  float *mean = sv + kMaxMembers * kLdp;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tiles = (n + 7) / 8;
+  for (int e = tid; e < kMaxMembers * kMaxMembers; e += kThreads) {
+    const int i = e / kMaxMembers, j = e - i * kMaxMembers;
+    g[i * kLdg + j] = i < n && j < n ? t4[i * n + j] : 0.0;
+  }
   const float dx2 = __fmul_rn(dx, dx), dt2 = __fmul_rn(dt, dt);
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < model;
-       p += (long long)gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int j = 0; j < n; j++) s = __fadd_rn(s, vels[j * model + p]);
-    const float mean = __fdiv_rn(s, (float)n);
-    // every member's A' t4 from the values before any of them is written
-    double t5s[kMaxMembers];
-    for (int i = 0; i < n; i++) {
-      double t5 = 0.0;
-      for (int j = 0; j < n; j++) t5 = fma((double)vels[j * model + p] - (double)mean, g[i * n + j], t5);
-      t5s[i] = t5;
+  for (long long p0 = (long long)blockIdx.x * kTile; p0 < model; p0 += (long long)gridDim.x * kTile) {
+    __syncthreads();
+    for (int e = tid; e < n * kTile; e += kThreads) {
+      const int j = e / kTile, k = e - j * kTile;
+      sv[j * kLdp + k] = p0 + k < model ? vels[j * model + p0 + k] : 1.0f;
     }
-    for (int i = 0; i < n; i++) {
-      const float vi = vels[i * model + p];
-      const float phys = __fsqrt_rn(__fdiv_rn(dx2, __fmul_rn(dt2, vi)));
-      const float upd = (float)((double)phys + t5s[i]);
-      vels[i * model + p] = __fdiv_rn(dx2, __fmul_rn(__fmul_rn(dt2, upd), upd));
+    __syncthreads();
+    if (tid < kTile) {
+      float s = 0.0f;
+#pragma unroll 8
+      for (int j = 0; j < n; j++) s = __fadd_rn(s, sv[j * kLdp + tid]);
+      mean[tid] = __fdiv_rn(s, (float)n);
+    }
+    __syncthreads();
+    // every member's A' t4 from the values before any of them is written:
+    // a warp reads and writes its own points only
+    const int pt = warp * 16 + (lane >> 2);
+    const double mu[2] = {(double)mean[pt], (double)mean[pt + 8]};
+    double acc[2][8][2] = {};
+    for (int k = 0; k < n; k += 4) {
+      const int j = k + (lane & 3);
+      double a[2];
+#pragma unroll
+      for (int t = 0; t < 2; t++) a[t] = j < n ? (double)sv[j * kLdp + pt + 8 * t] - mu[t] : 0.0;
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (i < tiles) {
+          const double b = g[(i * 8 + (lane >> 2)) * kLdg + j];
+          mma_f64(acc[0][i], a[0], b);
+          mma_f64(acc[1][i], a[1], b);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+          const int m = i * 8 + 2 * (lane & 3) + c;
+          if (m < n) {
+            float *v = sv + m * kLdp + pt + 8 * t;
+            const float phys = __fsqrt_rn(__fdiv_rn(dx2, __fmul_rn(dt2, *v)));
+            const float upd = (float)((double)phys + acc[t][i][c]);
+            *v = __fdiv_rn(dx2, __fmul_rn(__fmul_rn(dt2, upd), upd));
+          }
+        }
+    __syncthreads();
+    for (int e = tid; e < n * kTile; e += kThreads) {
+      const int j = e / kTile, k = e - j * kTile;
+      if (p0 + k < model) vels[j * model + p0 + k] = sv[j * kLdp + k];
     }
   }
 }
@@ -251,154 +353,227 @@ unsigned grid_of(long long n, int per) {
   return (unsigned)std::max(1LL, std::min(g, 4096LL));
 }
 
-// ---- the gain from the cross products, one CTA.  x = [X1 | X2 | X3],
-// each K x K row-major (K = kMaxMembers), first n x n used.
+// ---- the gain from the cross products.  x = [X1 | X2 | X3], each K x K
+// row-major (K = kMaxMembers), first n x n used.
 //
-// Eigenpairs of the symmetric X1 by two-sided Jacobi in the round-robin
-// (tournament) ordering: each round rotates n/2 disjoint index pairs at
-// once (all column rotations, then all row rotations: A <- J^T A J with J
-// the product of the round's plane rotations), n-1 rounds a sweep; a pair's
-// angle comes from its own 2 x 2 block, which no other rotation of the
-// round touches.  Sweeps stop when the off-diagonal square sum is at most
-// 1e-30 of the total (or after 100).  Eigenvalues sorted descending (ties
-// by index), s_k = sqrt(max(lambda_k, 0)), c = clipPosition(s)
-// (src/enfwi/Matrix.cpp:170-185), then
+// Eigenvalues of the symmetric X1 by two-sided Jacobi in the round-robin
+// (tournament) ordering, one CTA: each round rotates n/2 disjoint index
+// pairs at once, A <- J^T A J with J the product of the round's plane
+// rotations, n-1 rounds a sweep (n odd: one player idles, a zero row).
+// Sweeps stop when the off-diagonal square sum is at most 1e-30 of the
+// total (or after 100).  Eigenvalues sorted descending (ties by index),
+// s_k = sqrt(max(lambda_k, 0)), c = clipPosition(s)
+// (src/enfwi/Matrix.cpp:170-185).  The rotations go to `rot` and k_vectors
+// applies them to the rows of V, which do not depend on each other; then
 //   t4 = (X2 V_c diag(s^-4)) (V_c^T X3),  written column-major (the
 // reference's Matrix): t4[j*n + i] = row i, column j.
-// status[0] = c, status[1] = 1 if any cross product is not finite.
-constexpr int kGainThreads = 256;
-constexpr int kLd = kMaxMembers + 1;   // padded row stride in shared memory
+// status[0] = c, status[1] = 1 if any cross product is not finite,
+// status[2] = rounds.
+//
+// What bounds it is the chain of a round: a pair's angle (two reciprocal
+// roots in FP64), then everybody's rotation.  So A has two copies, read and
+// written in turn: while 496 threads rotate the 2 x 2 blocks of a round, one
+// a thread and the upper triangle only, the warp of the angles forms the
+// next round's off-diagonal elements itself from the same copy and goes on
+// to their angles; a round has one barrier.  Rows and columns are kept by
+// their place in the tournament (pair k's players at k and 32 + k), so that
+// a round moves every element by the same permutation and a thread's
+// addresses never change.  64 members: 0.39 ms, and 0.05 for V; 2.07 ms with
+// columns, rows, angles and V in turn in one CTA, 0.54 with one barrier but
+// player indices and the angle by square root and division.
+constexpr int kPairs = kMaxMembers / 2;
+constexpr int kBlocks = kPairs * (kPairs - 1) / 2;
+constexpr int kAngleWarp = (kBlocks + 31) / 32;
+constexpr int kGainThreads = (kAngleWarp + 1) * 32;
+constexpr int kLd = kMaxMembers + 1;   // the two rows that share a row of the triangle's storage
+constexpr int kTriangle = kMaxMembers * kLd / 2;
+constexpr int kMaxSweeps = 100;
+// rotations of at most kMaxSweeps, and the round formed ahead of the last
+constexpr int kMaxRotations = (kMaxSweeps * (kMaxMembers - 1) + 1) * kPairs;
 
-__host__ __device__ constexpr size_t gain_smem_bytes() {
-  return sizeof(double) * (3 * kMaxMembers * kLd + 4 * kMaxMembers + 2 * kGainThreads) +
-         sizeof(int) * (3 * kMaxMembers + 2 * (kMaxMembers / 2) + 4);
+// The players of pair k in the first round of m - 1, and of every sweep:
+// round r pairs (r + k, r - k) modulo m-1, pair 0 player m-1 with player r.
+// From a round to the next the player at place k (k > 0) moves to k - 1,
+// the one at 0 to 32 + 1, at 32 + k (k > 0) to 32 + k + 1, the last of
+// these to the last place k; the one at 32 stays.
+__device__ __forceinline__ int player_u(int k) { return k; }
+__device__ __forceinline__ int player_w(int k, int m) { return m - 1 - k; }
+__device__ __forceinline__ int place_next(int place, int half) {
+  if (half == 1 || place == kPairs) return place;
+  if (place < kPairs) return place == 0 ? kPairs + 1 : place - 1;
+  return place == kPairs + half - 1 ? half - 1 : place + 1;
 }
-
-__device__ double block_sum_fixed(double v, double *red) {
-  // fixed-order tree over the CTA's threads (deterministic)
-  red[threadIdx.x] = v;
-  __syncthreads();
-  for (int o = kGainThreads / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  const double r = red[0];
-  __syncthreads();
-  return r;
+__device__ __forceinline__ int place_before(int place, int half) {
+  if (half == 1 || place == kPairs) return place;
+  if (place < kPairs) return place == half - 1 ? kPairs + half - 1 : place + 1;
+  return place == kPairs + 1 ? 0 : place - 1;
+}
+// the same for the values of a pair's two players, one pair a lane
+__device__ __forceinline__ void pass_on(double &u, double &w, int lane, int half) {
+  const double up = __shfl_down_sync(0xffffffffu, u, 1);
+  const double dn = __shfl_up_sync(0xffffffffu, lane == 0 ? u : w, 1);
+  const double nu = half == 1 ? u : lane == half - 1 ? w : up;
+  w = lane == 0 ? w : dn;
+  u = nu;
+}
+// element (i, j) of the triangle, i != j: rows i and 63 - i share kLd doubles
+__device__ __forceinline__ int at(int i, int j) {
+  const int lo = min(i, j), hi = max(i, j);
+  return lo < kPairs ? lo * kLd + hi : (kMaxMembers - 1 - lo) * kLd + kMaxMembers - hi - 1;
 }
 
 __global__ void __launch_bounds__(kGainThreads)
-k_gain(double *t4, int *status, const double *x, int n) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double *A = reinterpret_cast<double *>(smem_raw);        // X1, then left = X2 V diag(s^-4)
-  double *V = A + kMaxMembers * kLd;                        // eigenvectors (columns)
-  double *R = V + kMaxMembers * kLd;                        // right = V^T X3
-  double *w = R + kMaxMembers * kLd;                        // eigenvalues
-  double *sv = w + kMaxMembers;                             // sorted singular values
-  double *cs = sv + kMaxMembers;                            // rotation cosines [n/2]
-  double *sn = cs + kMaxMembers;                            // rotation sines [n/2]
-  double *red = sn + kMaxMembers;                           // [2 * kGainThreads]
-  int *ord = reinterpret_cast<int *>(red + 2 * kGainThreads);
-  int *perm = ord + kMaxMembers;                            // tournament positions
-  int *pp = perm + kMaxMembers, *pq = pp + kMaxMembers / 2;
-  int *flag = pq + kMaxMembers / 2;
-  const int tid = threadIdx.x;
-  const int K = kMaxMembers;
-  const int m = (n + 1) & ~1;            // even number of tournament players (n odd: one idle)
-  const int half = m / 2;
+k_eigen(double2 *rot, double *sv_out, int *ord_out, int *status, const double *x, int n) {
+  __shared__ double A[2][kTriangle];
+  __shared__ double w[kMaxMembers], sv[kMaxMembers];
+  __shared__ double2 cs[2][kPairs];
+  __shared__ double red[2][kAngleWarp + 1];
+  __shared__ int ord[kMaxMembers], flag;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int K = kMaxMembers, m = (n + 1) & ~1, half = m / 2;
 
-  if (tid == 0) *flag = 0;
+  if (tid == 0) flag = 0;
+  for (int e = tid; e < 2 * kTriangle; e += kGainThreads) (&A[0][0])[e] = 0.0;
+  if (tid < K) w[tid] = 0.0;
   __syncthreads();
   for (int e = tid; e < n * n; e += kGainThreads) {
     const int i = e / n, j = e - i * n;
     const double a = x[i * K + j], b = x[K * K + i * K + j], c = x[2 * K * K + i * K + j];
-    if (!isfinite(a) || !isfinite(b) || !isfinite(c)) *flag = 1;
-    A[i * kLd + j] = a;
-    V[i * kLd + j] = i == j ? 1.0 : 0.0;
+    if (!isfinite(a) || !isfinite(b) || !isfinite(c)) flag = 1;
+    // player p's place
+    const int pi = i < half ? i : kPairs + m - 1 - i, pj = j < half ? j : kPairs + m - 1 - j;
+    if (i < j) A[0][at(pi, pj)] = a;
+    if (i == j) w[i] = a;
   }
   __syncthreads();
-  if (*flag) {
+  if (flag) {
     if (tid == 0) {
       status[0] = 0;
       status[1] = 1;
+      status[2] = 0;
     }
     return;
   }
 
-  for (int sweep = 0; sweep < 100; sweep++) {
-    double off = 0.0, tot = 0.0;
-    for (int e = tid; e < n * n; e += kGainThreads) {
-      const int i = e / n, j = e - i * n;
-      const double a = A[i * kLd + j];
-      tot += a * a;
-      if (i != j) off += a * a;
-    }
-    off = block_sum_fixed(off, red);
-    tot = block_sum_fixed(tot, red + kGainThreads);
-    if (off <= 1e-30 * tot || off == 0.0) break;
-    for (int round = 0; round < m - 1; round++) {
-      // pair k of this round: player m-1 meets player `round`, the others
-      // (round + k, round - k) modulo m-1
-      if (tid < half) {
-        int p, q;
-        if (tid == 0) {
-          p = round;
-          q = m - 1;
-        } else {
-          p = (round + tid) % (m - 1);
-          q = (round - tid + (m - 1)) % (m - 1);
-        }
-        if (p > q) {
-          const int t = p;
-          p = q;
-          q = t;
-        }
-        double c = 1.0, sg = 0.0;
-        if (q < n) {
-          const double apq = A[p * kLd + q];
-          if (apq != 0.0) {
-            const double theta = (A[q * kLd + q] - A[p * kLd + p]) / (2.0 * apq);
-            const double tt = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-            c = 1.0 / sqrt(tt * tt + 1.0);
-            sg = tt * c;
-          }
-        }
-        pp[tid] = p;
-        pq[tid] = q < n ? q : p;   // an idle player's pair rotates nothing
-        cs[tid] = c;
-        sn[tid] = q < n ? sg : 0.0;
-      }
-      __syncthreads();
-      // columns p, q of A and V
-      for (int e = tid; e < half * n; e += kGainThreads) {
-        const int k = e / half, pr = e - k * half;
-        const int p = pp[pr], q = pq[pr];
-        if (p == q) continue;
-        const double c = cs[pr], sg = sn[pr];
-        const double akp = A[k * kLd + p], akq = A[k * kLd + q];
-        A[k * kLd + p] = c * akp - sg * akq;
-        A[k * kLd + q] = sg * akp + c * akq;
-        const double vkp = V[k * kLd + p], vkq = V[k * kLd + q];
-        V[k * kLd + p] = c * vkp - sg * vkq;
-        V[k * kLd + q] = sg * vkp + c * vkq;
-      }
-      __syncthreads();
-      // rows p, q of A
-      for (int e = tid; e < half * n; e += kGainThreads) {
-        const int k = e / half, pr = e - k * half;
-        const int p = pp[pr], q = pq[pr];
-        if (p == q) continue;
-        const double c = cs[pr], sg = sn[pr];
-        const double apk = A[p * kLd + k], aqk = A[q * kLd + k];
-        A[p * kLd + k] = c * apk - sg * aqk;
-        A[q * kLd + k] = sg * apk + c * aqk;
-      }
-      __syncthreads();
+  // this thread's elements, read at f and written, a round on, at g: the
+  // block of pairs ba < bb; or (angles) the four that form the next
+  // element of pair `lane`
+  int ba = 0, bb = 0, f[4] = {}, g[4] = {}, own = 0;
+  bool su = false, sw = false;   // angles: the next players are their pairs' second now
+  const bool angles = warp == kAngleWarp && lane < half;
+  if (tid < half * (half - 1) / 2) {
+    int t = tid;
+    while (t >= half - 1 - ba) t -= half - 1 - ba++;
+    bb = ba + 1 + t;
+  }
+  const bool block = bb > 0;
+  if (angles) {
+    const int i = place_before(lane, half), j = place_before(kPairs + lane, half);
+    ba = i % kPairs;
+    bb = j % kPairs;
+    su = i >= kPairs;
+    sw = j >= kPairs;
+    own = half == 1 ? at(0, kPairs) : at(place_next(lane, half), place_next(kPairs + lane, half));
+  }
+  if (block || (angles && ba != bb)) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int i = ba + (e & 2 ? kPairs : 0), j = bb + (e & 1 ? kPairs : 0);
+      f[e] = at(i, j);
+      g[e] = at(place_next(i, half), place_next(j, half));
     }
   }
-  // descending order of the eigenvalues, ties by index
-  if (tid < n) w[tid] = A[tid * kLd + tid];
+
+  // the rotation of pair `lane` from its off-diagonal element o:
+  // cos 2 theta = |d| / h, h = sqrt(d^2 + 4 o^2), and c, s of the half angle.
+  // du, dw: the diagonal, which it moves
+  double du = 0.0, dw = 0.0;
+  auto angle = [&](double o, int buf, long long r) {
+    double c = 1.0, s = 0.0;
+    const double d = dw - du, o2 = 2.0 * o, h2 = fma(d, d, o2 * o2);
+    if (o != 0.0 && h2 > 0.0 && h2 < 1e300) {
+      const double rh = rsqrt(h2), y = 0.5 * rh, cc = fma(fabs(d), y, 0.5), rc = rsqrt(cc);
+      c = cc * rc;
+      s = (d >= 0.0 ? o2 : -o2) * y * rc;
+      const double t = s * rc;
+      du = fma(-t, o, du);
+      dw = fma(t, o, dw);
+    }
+    cs[buf][lane] = make_double2(c, s);
+    rot[r * kPairs + lane] = make_double2(c, s);
+  };
+  if (warp == kAngleWarp) {
+    if (angles) {
+      du = w[player_u(lane)];
+      dw = w[player_w(lane, m)];
+      angle(A[0][at(lane, kPairs + lane)], 0, 0);
+    }
+  }
+
+  int cur = 0;          // the copy to read
+  long long r = 0;      // rounds begun; angles are ready for this one
+  for (int sweep = 0; sweep < kMaxSweeps; sweep++) {
+    __syncthreads();
+    double off = 0.0, tot = 0.0;
+    for (int e = tid; e < kTriangle; e += kGainThreads) off += A[cur][e] * A[cur][e];
+    // the diagonal is a round ahead (the angles formed last): tot exceeds
+    // the total by no more than off
+    if (angles) tot = du * du + dw * dw;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    }
+    if (lane == 0) {
+      red[0][warp] = off;
+      red[1][warp] = tot;
+    }
+    __syncthreads();
+    off = 0.0;
+    for (int k = 0; k <= kAngleWarp; k++) off += red[0][k];
+    off *= 2.0;
+    tot = red[1][kAngleWarp] + off;
+    if (off <= 1e-30 * tot || off == 0.0) break;
+    for (int round = 0; round < m - 1; round++) {
+      const double *B = A[cur];
+      double *D = A[cur ^ 1];
+      const double2 *rc = cs[r & 1];
+      if (block) {
+        const double xpp = B[f[0]], xpq = B[f[1]], xqp = B[f[2]], xqq = B[f[3]];
+        const double2 ra = rc[ba], rb = rc[bb];
+        const double ypp = rb.x * xpp - rb.y * xpq, ypq = rb.y * xpp + rb.x * xpq;
+        const double yqp = rb.x * xqp - rb.y * xqq, yqq = rb.y * xqp + rb.x * xqq;
+        D[g[0]] = ra.x * ypp - ra.y * yqp;
+        D[g[2]] = ra.y * ypp + ra.x * yqp;
+        D[g[1]] = ra.x * ypq - ra.y * yqq;
+        D[g[3]] = ra.y * ypq + ra.x * yqq;
+      } else if (warp == kAngleWarp) {
+        double o = 0.0;
+        if (angles && ba != bb) {
+          const double2 ra = rc[ba], rb = rc[bb];
+          const double cb = sw ? rb.y : rb.x, sb = sw ? rb.x : -rb.y;
+          const double ca = su ? ra.y : ra.x, sa = su ? ra.x : -ra.y;
+          o = ca * (cb * B[f[0]] + sb * B[f[1]]) + sa * (cb * B[f[2]] + sb * B[f[3]]);
+        }
+        pass_on(du, dw, lane, half);
+        if (angles) {
+          D[own] = 0.0;   // the pair's own element is rotated to zero
+          angle(o, (r + 1) & 1, r + 1);
+        }
+      }
+      __syncthreads();
+      cur ^= 1;
+      r++;
+    }
+  }
+  // round r, formed ahead, is in the diagonal and goes into V; in A it would
+  // move elements that are at rounding level.  Places are the first round's
+  if (angles) {
+    w[player_u(lane)] = du;
+    w[player_w(lane, m)] = dw;
+  }
   __syncthreads();
+  // descending order of the eigenvalues, ties by index
   if (tid < n) {
     int rank = 0;
     const double wi = w[tid];
@@ -406,7 +581,11 @@ k_gain(double *t4, int *status, const double *x, int n) {
     ord[rank] = tid;
   }
   __syncthreads();
-  if (tid < n) sv[tid] = sqrt(fmax(w[ord[tid]], 0.0));
+  if (tid < n) {
+    sv[tid] = sqrt(fmax(w[ord[tid]], 0.0));
+    sv_out[tid] = sv[tid];
+    ord_out[tid] = ord[tid];
+  }
   __syncthreads();
   if (tid == 0) {
     // clipPosition (Matrix.cpp:170-185); relativeError is a float literal
@@ -417,83 +596,191 @@ k_gain(double *t4, int *status, const double *x, int n) {
       sum += fabs(sv[pos]);
       if (rel / (1 - rel) * sum > (n - pos + 1) * sv[pos + 1]) break;
     }
-    flag[0] = pos + 1;
-  }
-  __syncthreads();
-  const int c = flag[0];
-  // left[i][k] = (X2 V)[i][ord[k]] s_k^-4 (into A); right[k][i] = (V^T X3)[ord[k]][i]
-  for (int e = tid; e < n * c; e += kGainThreads) {
-    const int i = e / c, k = e - i * c;
-    const int col = ord[k];
-    double l = 0.0, r = 0.0;
-    for (int j = 0; j < n; j++) {
-      l += x[K * K + i * K + j] * V[j * kLd + col];
-      r += V[j * kLd + col] * x[2 * K * K + j * K + i];
-    }
-    const double s2 = sv[k] * sv[k];
-    A[i * kLd + k] = l * (1.0 / (s2 * s2));
-    R[k * kLd + i] = r;
-  }
-  __syncthreads();
-  for (int e = tid; e < n * n; e += kGainThreads) {
-    const int j = e / n, i = e - j * n;
-    double acc = 0.0;
-    for (int k = 0; k < c; k++) acc += A[i * kLd + k] * R[k * kLd + j];
-    t4[j * n + i] = acc;
-  }
-  if (tid == 0) {
-    status[0] = c;
+    status[0] = pos + 1;
     status[1] = 0;
+    status[2] = (int)r + 1;
   }
 }
 
+// Row blockIdx.x of V = the product of the rotations, one warp: lane k holds
+// the row's entries of pair k's two players and passes them on.  A round is
+// two dependent operations and a shuffle; its rotations are loaded 8 to 16
+// rounds ahead.
+__global__ void __launch_bounds__(32) k_vectors(double *v, const double2 *rot, const int *status, int n) {
+  const int row = blockIdx.x, lane = threadIdx.x, m = (n + 1) & ~1, half = m / 2;
+  const int rounds = status[2];
+  if (status[1]) return;
+  constexpr int kAhead = 8;
+  double2 c[kAhead], next[kAhead];
+  const double2 *from = rot + min(lane, half - 1);
+  auto load = [&](double2 (&x)[kAhead], int r) {
+#pragma unroll
+    for (int e = 0; e < kAhead; e++) x[e] = from[(long long)min(r + e, rounds - 1) * kPairs];
+  };
+  double u = player_u(lane) == row ? 1.0 : 0.0, w = player_w(lane, m) == row ? 1.0 : 0.0;
+  if (lane >= half) u = w = 0.0;
+  load(c, 0);
+  for (int r = 0; r < rounds; r += kAhead) {
+    load(next, r + kAhead);
+#pragma unroll
+    for (int e = 0; e < kAhead; e++)
+      if (r + e < rounds) {
+        if (r + e > 0) pass_on(u, w, lane, half);
+        const double nu = c[e].x * u - c[e].y * w;
+        w = c[e].y * u + c[e].x * w;
+        u = nu;
+      }
+#pragma unroll
+    for (int e = 0; e < kAhead; e++) c[e] = next[e];
+  }
+  // the last rotation is the first of a sweep: places are the first round's
+  if (lane < half) {
+    v[row * kMaxMembers + player_u(lane)] = u;
+    v[row * kMaxMembers + player_w(lane, m)] = w;
+  }
+}
+
+// left[i][k] = (X2 V)[i][ord[k]] s_k^-4 (first 64 threads, i = blockIdx.x);
+// right[k][i] = (V^T X3)[ord[k]][i] (the others, k = blockIdx.x)
+__global__ void __launch_bounds__(2 * kMaxMembers)
+k_sides(double *left, double *right, const double *x, const double *v, const double *sv, const int *ord,
+        const int *status, int n) {
+  const int K = kMaxMembers, c = status[0], b = blockIdx.x, t = threadIdx.x % kMaxMembers;
+  if (status[1]) return;
+  if (threadIdx.x < kMaxMembers) {
+    if (t >= c) return;
+    const int col = ord[t];
+    double l = 0.0;
+#pragma unroll 8
+    for (int j = 0; j < n; j++) l += x[K * K + b * K + j] * v[j * K + col];
+    const double s2 = sv[t] * sv[t];
+    left[b * K + t] = l * (1.0 / (s2 * s2));
+  } else {
+    if (b >= c || t >= n) return;
+    const int col = ord[b];
+    double r = 0.0;
+#pragma unroll 8
+    for (int j = 0; j < n; j++) r += v[j * K + col] * x[2 * K * K + j * K + t];
+    right[b * K + t] = r;
+  }
+}
+
+// row i = threadIdx.x, column j = blockIdx.x of t4
+__global__ void __launch_bounds__(kMaxMembers)
+k_gain(double *t4, const double *left, const double *right, const int *status, int n) {
+  const int K = kMaxMembers, i = threadIdx.x, j = blockIdx.x, c = status[0];
+  if (status[1] || i >= n) return;
+  double acc = 0.0;
+#pragma unroll 8
+  for (int k = 0; k < c; k++) acc += left[i * K + k] * right[k * K + j];
+  t4[j * n + i] = acc;
+}
+
 // Device memory of one analysis, held by the caller until its results are
-// back (freeing it earlier would synchronise the device mid-analysis).
+// back.  The results come first: sigma, status ([0] clip, [1] non-finite
+// cross products, [2] rounds), t4.
 struct GainScratch {
-  DevBuf<unsigned long long> best;
-  DevBuf<double> sigma, partials, x, t4;
-  DevBuf<int> status;   // [0] clip, [1] non-finite cross products
+  static constexpr size_t kSquare = (size_t)kMaxMembers * kMaxMembers;
+  static constexpr int kResults = 3;   // doubles before t4
+  static constexpr size_t bytes(int nparts) {
+    return sizeof(double) * (kResults + 1 + 7 * kSquare + 2 * kMaxMembers + 2 * (size_t)kMaxRotations +
+                             nparts * 3 * kSquare);
+  }
+  Scratch mem;
+  double *sigma, *t4, *x, *v, *left, *right, *sv, *partials;
+  int *status, *ord;
+  double2 *rot;
+  unsigned long long *best;
+
+  explicit GainScratch(int nparts) : mem(bytes(nparts)) {
+    double *p = static_cast<double *>(mem.get());
+    auto take = [&p](size_t doubles) {
+      double *q = p;
+      p += doubles;
+      return q;
+    };
+    sigma = take(1);
+    status = reinterpret_cast<int *>(take(2));
+    t4 = take(kSquare);
+    best = reinterpret_cast<unsigned long long *>(take(1));   // rot below: 16-byte aligned
+    rot = reinterpret_cast<double2 *>(take(2 * (size_t)kMaxRotations));
+    x = take(3 * kSquare);
+    v = take(kSquare);
+    left = take(kSquare);
+    right = take(kSquare);
+    sv = take(kMaxMembers);
+    ord = reinterpret_cast<int *>(take(kMaxMembers));
+    partials = take(nparts * 3 * kSquare);
+  }
 };
+
+int cross_parts(long long rows) {
+  int dev = 0, sms = 148;
+  SWFWI_CUDA(cudaGetDevice(&dev));
+  SWFWI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  return (int)std::min<long long>((rows + kRows - 1) / kRows, sms);
+}
 
 // The analysis's device part: sigma (first call), cross products, gain into
 // sc.t4 [n*n] (column-major), sc.status, sc.sigma.
 void gain_on_device(const float *hona, const float *dobs, const double *z, long long rows, int n, float sigfac,
-                    double sigma_in, unsigned long long seed, GainScratch &sc, cudaStream_t st) {
-  sc.sigma.resize(1);
-  sc.t4.resize((size_t)n * n);
-  sc.status.resize(2);
-  if (!(sigma_in > 0.0)) {
+                    const double *sigma_in, unsigned long long seed, int nparts, GainScratch &sc, cudaStream_t st) {
+  if (!(*sigma_in > 0.0)) {
     // initPerturbation's first call: sigma = max|HA'| * sigmaFactor
-    sc.best.resize(1);
-    SWFWI_CUDA(cudaMemsetAsync(sc.best.get(), 0, sizeof(unsigned long long), st));
-    k_maxkey<<<grid_of(rows, kThreads), kThreads, 0, st>>>(sc.best.get(), hona, rows, n);
+    SWFWI_CUDA(cudaMemsetAsync(sc.best, 0, sizeof(unsigned long long), st));
+    k_maxkey<<<grid_of(rows, kThreads), kThreads, 0, st>>>(sc.best, hona, rows, n);
     note_launch();
-    k_value_at<<<1, 1, 0, st>>>(sc.sigma.get(), sc.best.get(), hona, rows, n, sigfac);
+    k_value_at<<<1, 1, 0, st>>>(sc.sigma, sc.best, hona, rows, n, sigfac);
     note_launch();
   } else {
-    SWFWI_CUDA(cudaMemcpyAsync(sc.sigma.get(), &sigma_in, sizeof(double), cudaMemcpyHostToDevice, st));
+    SWFWI_CUDA(cudaMemcpyAsync(sc.sigma, sigma_in, sizeof(double), cudaMemcpyHostToDevice, st));
   }
-  int dev = 0, sms = 148;
-  SWFWI_CUDA(cudaGetDevice(&dev));
-  SWFWI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const long long chunks = (rows + kRowsPerChunk - 1) / kRowsPerChunk;
-  const int nparts = (int)std::min<long long>(chunks, 2LL * sms);
-  const int m = 3 * kMaxMembers * kMaxMembers;
-  sc.partials.resize((size_t)nparts * m);
-  sc.x.resize(m);
+  // once each (thread-safe static init)
+  static const cudaError_t attr_z = cudaFuncSetAttribute(k_cross<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)cross_smem_bytes());
+  static const cudaError_t attr_d = cudaFuncSetAttribute(k_cross<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)cross_smem_bytes());
+  SWFWI_CUDA(attr_z);
+  SWFWI_CUDA(attr_d);
   if (z)
-    k_cross<false><<<nparts, kThreads, 0, st>>>(sc.partials.get(), hona, dobs, z, rows, n, sc.sigma.get(), seed);
+    k_cross<false><<<nparts, kCrossThreads, cross_smem_bytes(), st>>>(sc.partials, hona, dobs, z, rows, n, sc.sigma,
+                                                                      seed);
   else
-    k_cross<true><<<nparts, kThreads, 0, st>>>(sc.partials.get(), hona, dobs, nullptr, rows, n, sc.sigma.get(),
-                                               seed);
+    k_cross<true><<<nparts, kCrossThreads, cross_smem_bytes(), st>>>(sc.partials, hona, dobs, nullptr, rows, n,
+                                                                     sc.sigma, seed);
   note_launch();
-  k_sum_partials<<<(m + 255) / 256, 256, 0, st>>>(sc.x.get(), sc.partials.get(), nparts);
+  k_sum_partials<<<3 * kMaxMembers * kMaxMembers / 64, 64, 0, st>>>(sc.x, sc.partials, nparts);
   note_launch();
-  // once (thread-safe static init)
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_gain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gain_smem_bytes());
-  SWFWI_CUDA(attr);
-  k_gain<<<1, kGainThreads, gain_smem_bytes(), st>>>(sc.t4.get(), sc.status.get(), sc.x.get(), n);
+  k_eigen<<<1, kGainThreads, 0, st>>>(sc.rot, sc.sv, sc.ord, sc.status, sc.x, n);
+  note_launch();
+  k_vectors<<<n, 32, 0, st>>>(sc.v, sc.rot, sc.status, n);
+  note_launch();
+  k_sides<<<n, 2 * kMaxMembers, 0, st>>>(sc.left, sc.right, sc.x, sc.v, sc.sv, sc.ord, sc.status, n);
+  note_launch();
+  k_gain<<<n, kMaxMembers, 0, st>>>(sc.t4, sc.left, sc.right, sc.status, n);
+  note_launch();
+  SWFWI_CUDA(cudaGetLastError());
+}
+
+// sigma, clip and (unless null) t4 to the host, in one copy
+void fetch_gain(GainScratch &sc, int n, double *sigma, double *t4, int *clip, cudaStream_t st) {
+  std::vector<double> h(GainScratch::kResults + (t4 ? (size_t)n * n : 0));
+  SWFWI_CUDA(cudaMemcpyAsync(h.data(), sc.sigma, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st));
+  SWFWI_CUDA(cudaStreamSynchronize(st));
+  sc.mem.idle();
+  int hs[2];
+  std::memcpy(hs, &h[1], sizeof(hs));
+  *sigma = h[0];
+  if (t4) std::memcpy(t4, &h[GainScratch::kResults], sizeof(double) * n * n);
+  if (hs[1]) throw Error(SWFWI_ERR_NONFINITE, "non-finite data in the analysis");
+  if (clip) *clip = hs[0];
+}
+
+template <typename F, typename... Args>
+void launch_update(F kernel, long long model, cudaStream_t st, Args... args) {
+  SWFWI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem_bytes()));
+  kernel<<<(unsigned)std::min<long long>((model + kTile - 1) / kTile, 444), kThreads, update_smem_bytes(), st>>>(
+      args...);
   note_launch();
   SWFWI_CUDA(cudaGetLastError());
 }
@@ -511,15 +798,10 @@ extern "C" int swfwi_enkf_gain_matrix(const float *hona, const float *dobs, cons
     SWFWI_REQUIRE(n >= 2 && n <= kMaxMembers, "members must be 2..64");
     SWFWI_REQUIRE(rows > 0 && rows * n < 0xFFFFFFFFLL, "rows x members must be below 2^32");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    GainScratch sc;
-    gain_on_device(hona, dobs, z, rows, n, sigfac, *sigma, seed, sc, st);
-    int hs[2] = {0, 0};
-    SWFWI_CUDA(cudaMemcpyAsync(hs, sc.status.get(), sizeof(hs), cudaMemcpyDeviceToHost, st));
-    SWFWI_CUDA(cudaMemcpyAsync(sigma, sc.sigma.get(), sizeof(double), cudaMemcpyDeviceToHost, st));
-    SWFWI_CUDA(cudaMemcpyAsync(t4, sc.t4.get(), sizeof(double) * n * n, cudaMemcpyDeviceToHost, st));
-    SWFWI_CUDA(cudaStreamSynchronize(st));
-    if (hs[1]) throw Error(SWFWI_ERR_NONFINITE, "non-finite data in the analysis");
-    if (clip) *clip = hs[0];
+    const int nparts = cross_parts(rows);
+    GainScratch sc(nparts);
+    gain_on_device(hona, dobs, z, rows, n, sigfac, sigma, seed, nparts, sc, st);
+    fetch_gain(sc, n, sigma, t4, clip, st);
   });
 }
 
@@ -532,22 +814,14 @@ extern "C" int swfwi_enkf_analyze(const float *hona, const float *dobs, const do
     SWFWI_REQUIRE(n >= 2 && n <= kMaxMembers, "members must be 2..64");
     SWFWI_REQUIRE(rows > 0 && rows * n < 0xFFFFFFFFLL, "rows x members must be below 2^32");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    GainScratch sc;
-    gain_on_device(hona, dobs, z, rows, n, sigfac, *sigma, seed, sc, st);
+    const int nparts = cross_parts(rows);
+    GainScratch sc(nparts);
+    gain_on_device(hona, dobs, z, rows, n, sigfac, sigma, seed, nparts, sc, st);
     // a non-finite gain leaves the members unchanged: the update skips when
     // status[1] is set
-    k_update_guarded<<<grid_of(model_size, kThreads), kThreads, 0, st>>>(vels, model_size, n, sc.t4.get(), dx, dt,
-                                                                         sc.status.get());
-    note_launch();
-    SWFWI_CUDA(cudaGetLastError());
-    int hs[2] = {0, 0};
-    SWFWI_CUDA(cudaMemcpyAsync(hs, sc.status.get(), sizeof(hs), cudaMemcpyDeviceToHost, st));
-    SWFWI_CUDA(cudaMemcpyAsync(sigma, sc.sigma.get(), sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (t4_out)
-      SWFWI_CUDA(cudaMemcpyAsync(t4_out, sc.t4.get(), sizeof(double) * n * n, cudaMemcpyDeviceToHost, st));
-    SWFWI_CUDA(cudaStreamSynchronize(st));
-    if (hs[1]) throw Error(SWFWI_ERR_NONFINITE, "non-finite data in the analysis");
-    if (clip) *clip = hs[0];
+    launch_update(k_update_guarded, model_size, st, vels, model_size, n, (const double *)sc.t4, dx, dt,
+                  (const int *)sc.status);
+    fetch_gain(sc, n, sigma, t4_out, clip, st);
   });
 }
 
@@ -557,12 +831,11 @@ extern "C" int swfwi_enkf_update(float *vels, long long model_size, int n, const
     SWFWI_REQUIRE(vels && t4 && model_size > 0, "bad update arguments");
     SWFWI_REQUIRE(n >= 2 && n <= kMaxMembers, "members must be 2..64");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    DevBuf<double> g((size_t)n * n);
+    Scratch g(sizeof(double) * n * n);
     SWFWI_CUDA(cudaMemcpyAsync(g.get(), t4, sizeof(double) * n * n, cudaMemcpyHostToDevice, st));
-    k_update<<<grid_of(model_size, kThreads), kThreads, 0, st>>>(vels, model_size, n, g.get(), dx, dt);
-    note_launch();
-    SWFWI_CUDA(cudaGetLastError());
+    launch_update(k_update, model_size, st, vels, model_size, n, static_cast<const double *>(g.get()), dx, dt);
     SWFWI_CUDA(cudaStreamSynchronize(st));
+    g.idle();
   });
 }
 
