@@ -17,6 +17,8 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 constexpr int kEw = 256;   // threads of the elementwise kernels
+constexpr int kDotThreads = 32;    // of the channel sums: kEw / C runs x C / 8 groups
+constexpr int kRowThreads = 128;   // threads of those that take an image row a blockIdx.y
 
 inline void noted() { g_kernel_launches.fetch_add(1, std::memory_order_relaxed); }
 inline unsigned blocks_for(long long n, int threads = kEw) {
@@ -577,15 +579,43 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const bf16 *__restrict__ dz, i
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// out[i] = sum over r = 0..rows-1, in order, of part[r * len + i]
-__global__ void k_reduce_rows(const float *__restrict__ part, int rows, long long len,
-                              float *__restrict__ out) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < len;
-       i += (long long)gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int r = 0; r < rows; r++) s += part[(long long)r * len + i];
-    out[i] = s;
+// Sums of partials, two sets a launch: out[i] = sum over r = 0..rows-1, in
+// order, of part[r * len + i].  A block takes 32 columns: its warps fetch 128
+// rows at a time into shared memory, one of them adds the rows.  (With a
+// column a thread, 9 blocks of loads in turn, 437 rows of 2304 columns took
+// 49 us and the 256 rows of a bias 23.)
+struct RowSum {
+  const float *part;
+  int rows;
+  long long len;
+  float *out;
+};
+constexpr int kSumRows = 128;
+__global__ void __launch_bounds__(kEw) k_reduce_rows(RowSum a, RowSum b, unsigned ablocks) {
+  __shared__ float buf[2][kSumRows][32];
+  const RowSum &x = blockIdx.x < ablocks ? a : b;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long i = (long long)(blockIdx.x < ablocks ? blockIdx.x : blockIdx.x - ablocks) * 32 + lane;
+  const bool in = i < x.len;
+  auto fetch = [&](int r0, float (*to)[32]) {
+#pragma unroll
+    for (int k = 0; k < kSumRows / 8; k++) {
+      const int r = r0 + warp + 8 * k;
+      to[warp + 8 * k][lane] = in && r < x.rows ? x.part[(long long)r * x.len + i] : 0.0f;
+    }
+  };
+  float s = 0.0f;
+  fetch(0, buf[0]);
+  for (int r0 = 0, k = 0; r0 < x.rows; r0 += kSumRows, k ^= 1) {
+    __syncthreads();
+    if (r0 + kSumRows < x.rows) fetch(r0 + kSumRows, buf[k ^ 1]);
+    if (warp == 0) {
+      const int m = min(kSumRows, x.rows - r0);
+#pragma unroll 16
+      for (int r = 0; r < m; r++) s += buf[k][r][lane];
+    }
   }
+  if (warp == 0 && in) x.out[i] = s;
 }
 
 // --------------------------------------------------------- elementwise parts
@@ -627,73 +657,84 @@ __global__ void k_pool(const bf16 *__restrict__ in, bf16 *__restrict__ out, int 
   }
 }
 
-// din (fine grid) += 0.25 dout (coarse grid)
-__global__ void k_pool_bwd(const float *__restrict__ dout, float *__restrict__ din, int N, int H,
-                           int W, int C) {
-  const long long total = (long long)N * H * W * C;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(e % C);
-    long long q = e / C;
-    const int w = (int)(q % W);
-    q /= W;
-    const int h = (int)(q % H);
-    const int n = (int)(q / H);
-    din[e] += 0.25f * dout[((long long)(n * (H / 2) + h / 2) * (W / 2) + w / 2) * C + c];
-  }
+// 8 channels of a pixel: 16 bytes BF16, 32 bytes FP32
+struct alignas(16) F8 {
+  float4 a, b;
+};
+__device__ __forceinline__ F8 ld8(const float *p) {
+  return {*reinterpret_cast<const float4 *>(p), *reinterpret_cast<const float4 *>(p + 4)};
+}
+__device__ __forceinline__ float lo_f(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
+
+// cat[n][h][w] = (low[n][h/2][w/2][0..C1), skip[n][h][w][0..C2)), 16 bytes a
+// thread, an image row a blockIdx.y
+__global__ void __launch_bounds__(kRowThreads)
+k_upcat(const bf16 *__restrict__ low, int C1, const bf16 *__restrict__ skip, int C2, bf16 *__restrict__ cat, int H,
+        int W) {
+  const int g1 = C1 / 8, g2 = C2 / 8, gt = g1 + g2;
+  const int e = blockIdx.x * kRowThreads + threadIdx.x, row = blockIdx.y;
+  if (e >= W * gt) return;
+  const int w = e / gt, g = e - w * gt, n = row / H, h = row - n * H;
+  const uint4 *src = g < g1 ? reinterpret_cast<const uint4 *>(low) +
+                                  ((long long)(n * (H / 2) + h / 2) * (W / 2) + w / 2) * g1 + g
+                            : reinterpret_cast<const uint4 *>(skip) + ((long long)row * W + w) * g2 + g - g1;
+  reinterpret_cast<uint4 *>(cat)[(long long)row * W * gt + e] = *src;
 }
 
-// cat[n][h][w] = (low[n][h/2][w/2][0..C1), skip[n][h][w][0..C2))
-__global__ void k_upcat(const bf16 *__restrict__ low, int C1, const bf16 *__restrict__ skip, int C2,
-                        bf16 *__restrict__ cat, int N, int H, int W) {
-  const int Ct = C1 + C2, cp = Ct / 2;
-  const long long total = (long long)N * H * W * cp;
-  const uint32_t *lo = reinterpret_cast<const uint32_t *>(low);
-  const uint32_t *sk = reinterpret_cast<const uint32_t *>(skip);
-  uint32_t *o = reinterpret_cast<uint32_t *>(cat);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int c = 2 * (int)(e % cp);
-    const long long pix = e / cp;
-    const int w = (int)(pix % W);
-    const long long nh = pix / W;
-    const int h = (int)(nh % H);
-    const int n = (int)(nh / H);
-    uint32_t v;
-    if (c < C1) v = lo[(((long long)(n * (H / 2) + h / 2) * (W / 2) + w / 2) * C1 + c) / 2];
-    else v = sk[(pix * C2 + (c - C1)) / 2];
-    o[e] = v;
+// ReLU gradient of a layer, rounded to BF16 for the tensor-core products:
+// dz = y > 0 ? dY : 0, 8 channels a thread, an image row a blockIdx.y.  Where
+// dY is a plain function of other gradients it is formed here and never
+// stored: kPlain: a is dY; kLow: the four fine gradients (a: dcat, of Ct
+// channels) of an upsampled pixel; kSkip: the skip's share of a concatenation
+// (channels C1.. of a) plus a quarter of the pooled gradient b; kOut: the
+// output layer's, a[pixel] times b[channel].
+enum { kPlain, kLow, kSkip, kOut };
+template <int MODE>
+__global__ void __launch_bounds__(kRowThreads)
+k_relu_mask(const float *__restrict__ a, const float *__restrict__ b, int Ct, int C1, const bf16 *__restrict__ y,
+            bf16 *__restrict__ dz, int H, int W, int C) {
+  const int g8 = C / 8, e = blockIdx.x * kRowThreads + threadIdx.x, row = blockIdx.y;
+  if (e >= W * g8) return;
+  const int w = e / g8, c = (e - w * g8) * 8;
+  const long long p = (long long)row * W + w;
+  float v[8];
+  auto put = [&](const F8 &x) {
+    v[0] = x.a.x; v[1] = x.a.y; v[2] = x.a.z; v[3] = x.a.w;
+    v[4] = x.b.x; v[5] = x.b.y; v[6] = x.b.z; v[7] = x.b.w;
+  };
+  auto add = [&](const F8 &x) {
+    v[0] += x.a.x; v[1] += x.a.y; v[2] += x.a.z; v[3] += x.a.w;
+    v[4] += x.b.x; v[5] += x.b.y; v[6] += x.b.z; v[7] += x.b.w;
+  };
+  if constexpr (MODE == kPlain) {
+    put(ld8(a + p * C + c));
+  } else if constexpr (MODE == kLow) {
+    // pixel rows of the fine grid are 2 * row and the next: 2 n H + 2 h
+    const float *r0 = a + (((long long)row * 2) * (2 * W) + 2 * w) * Ct + c, *r1 = r0 + (long long)2 * W * Ct;
+    put(ld8(r0));
+    add(ld8(r0 + Ct));
+    add(ld8(r1));
+    add(ld8(r1 + Ct));
+  } else if constexpr (MODE == kSkip) {
+    const int n = row / H, h = row - n * H;
+    put(ld8(a + p * Ct + C1 + c));
+    F8 q = ld8(b + ((long long)(n * (H / 2) + h / 2) * (W / 2) + w / 2) * C + c);
+    q.a.x *= 0.25f; q.a.y *= 0.25f; q.a.z *= 0.25f; q.a.w *= 0.25f;
+    q.b.x *= 0.25f; q.b.y *= 0.25f; q.b.z *= 0.25f; q.b.w *= 0.25f;
+    add(q);
+  } else {
+    const float d = a[p];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = d * b[c + k];
   }
-}
-
-// dlow[n][h][w][c] = sum of the four fine gradients of its copies
-__global__ void k_upcat_bwd_low(const float *__restrict__ dcat, int Ct, int C1, float *__restrict__ dlow,
-                                int N, int Hl, int Wl) {
-  const long long total = (long long)N * Hl * Wl * C1;
-  const int H = 2 * Hl, W = 2 * Wl;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(e % C1);
-    long long q = e / C1;
-    const int w = (int)(q % Wl);
-    q /= Wl;
-    const int h = (int)(q % Hl);
-    const int n = (int)(q / Hl);
-    const long long r0 = ((long long)(n * H + 2 * h) * W + 2 * w) * Ct + c;
-    const long long r1 = r0 + (long long)W * Ct;
-    dlow[e] = ((dcat[r0] + dcat[r0 + Ct]) + dcat[r1]) + dcat[r1 + Ct];
-  }
-}
-
-__global__ void k_upcat_bwd_skip(const float *__restrict__ dcat, int Ct, int C1, float *__restrict__ dskip,
-                                 long long P, int C2) {
-  const long long total = P * C2;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long p = e / C2;
-    const int c = (int)(e - p * C2);
-    dskip[e] = dcat[p * Ct + C1 + c];
-  }
+  const uint4 m = *reinterpret_cast<const uint4 *>(y + p * C + c);
+  uint4 o;
+  o.x = pack_bf16(lo_f(m.x) > 0.0f ? v[0] : 0.0f, hi_f(m.x) > 0.0f ? v[1] : 0.0f);
+  o.y = pack_bf16(lo_f(m.y) > 0.0f ? v[2] : 0.0f, hi_f(m.y) > 0.0f ? v[3] : 0.0f);
+  o.z = pack_bf16(lo_f(m.z) > 0.0f ? v[4] : 0.0f, hi_f(m.z) > 0.0f ? v[5] : 0.0f);
+  o.w = pack_bf16(lo_f(m.w) > 0.0f ? v[6] : 0.0f, hi_f(m.w) > 0.0f ? v[7] : 0.0f);
+  *reinterpret_cast<uint4 *>(dz + p * C + c) = o;
 }
 
 // y[p] = b + sum_c w[c] u[p][c]   (FP32)
@@ -702,38 +743,64 @@ __global__ void k_out_fwd(const bf16 *__restrict__ u, const float *__restrict__ 
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P;
        p += (long long)gridDim.x * blockDim.x) {
     float s = 0.0f;
-    for (int c = 0; c < C; c++) s = fmaf(w[c], __bfloat162float(u[p * C + c]), s);
+    for (int c = 0; c < C; c += 8) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(u + p * C + c);
+      s = fmaf(w[c], lo_f(v.x), s);
+      s = fmaf(w[c + 1], hi_f(v.x), s);
+      s = fmaf(w[c + 2], lo_f(v.y), s);
+      s = fmaf(w[c + 3], hi_f(v.y), s);
+      s = fmaf(w[c + 4], lo_f(v.z), s);
+      s = fmaf(w[c + 5], hi_f(v.z), s);
+      s = fmaf(w[c + 6], lo_f(v.w), s);
+      s = fmaf(w[c + 7], hi_f(v.w), s);
+    }
     y[p] = s + b[0];
   }
 }
 
-__global__ void k_out_bwd_dx(const float *__restrict__ dy, const float *__restrict__ w,
-                             float *__restrict__ du, long long P, int C) {
-  const long long total = P * C;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long p = e / C;
-    du[e] = dy[p] * w[e - p * C];
+// part[slot][c] = sum over the slot's pixels of a[p][c] * (WGT ? wgt[p] : 1):
+// slot s of kRedBlocks has `runs` = kEw / C runs, run k the pixels
+// s * runs + k, + kRedBlocks * runs, ..., added in order and then run by run.
+// 8 channels a thread and 16 loads in flight; the slots are summed by
+// k_reduce_rows.  39 MB (16 channels of 480 x 160 x 16 pixels) in 2-byte loads
+// took 78 us.
+template <bool WGT>
+__global__ void __launch_bounds__(kDotThreads) k_chan_dot(const bf16 *__restrict__ a, const float *__restrict__ wgt,
+                                                          long long P, int C, float *__restrict__ part) {
+  __shared__ float red[kEw];   // [run][C]: C * runs <= kEw
+  const int g8 = C / 8, runs = kEw / C, run = threadIdx.x / g8, c = (threadIdx.x - run * g8) * 8;
+  if (run < runs) {
+    float s[8] = {};
+    const long long step = (long long)gridDim.x * runs;
+    constexpr int kDeep = 16;
+    for (long long p0 = (long long)blockIdx.x * runs + run; p0 < P; p0 += kDeep * step) {
+      uint4 v[kDeep];
+      float f[kDeep];
+#pragma unroll
+      for (int k = 0; k < kDeep; k++) {
+        const long long p = p0 + k * step;
+        v[k] = p < P ? *reinterpret_cast<const uint4 *>(a + p * C + c) : make_uint4(0u, 0u, 0u, 0u);
+        f[k] = WGT && p < P ? wgt[p] : 0.0f;
+      }
+#pragma unroll
+      for (int k = 0; k < kDeep; k++) {
+        if (p0 + k * step >= P) break;
+        const uint32_t q[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          s[2 * h] = WGT ? fmaf(lo_f(q[h]), f[k], s[2 * h]) : s[2 * h] + lo_f(q[h]);
+          s[2 * h + 1] = WGT ? fmaf(hi_f(q[h]), f[k], s[2 * h + 1]) : s[2 * h + 1] + hi_f(q[h]);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) red[run * C + c + k] = s[k];
   }
-}
-
-// part[block][c] = sum over the block's pixels of a[p][c] * (wgt ? wgt[p] :
-// 1); C divides the block size.  Summed over blocks by k_reduce_rows.
-__global__ void k_chan_dot(const bf16 *__restrict__ a, const float *__restrict__ wgt, long long P,
-                           int C, float *__restrict__ part) {
-  __shared__ float red[kEw];
-  const int c = threadIdx.x % C, lp = threadIdx.x / C, ps = kEw / C;
-  float s = 0.0f;
-  for (long long p = (long long)blockIdx.x * ps + lp; p < P; p += (long long)gridDim.x * ps) {
-    const float v = __bfloat162float(a[p * C + c]);
-    s += wgt ? v * wgt[p] : v;
-  }
-  red[threadIdx.x] = s;
   __syncthreads();
-  if (threadIdx.x < C) {
-    float tsum = 0.0f;
-    for (int k = 0; k < ps; k++) tsum += red[k * C + threadIdx.x];
-    part[(long long)blockIdx.x * C + threadIdx.x] = tsum;
+  for (int k = threadIdx.x; k < C; k += kDotThreads) {
+    float t = 0.0f;
+    for (int r = 0; r < runs; r++) t += red[r * C + k];
+    part[(long long)blockIdx.x * C + k] = t;
   }
 }
 
@@ -764,16 +831,15 @@ __global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, 
     dy[p] = scale * r;
     s += (double)r * r;
   }
+  // one addition to the loss a block
+  __shared__ double red[kEw / 32];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, s);
-}
-
-// ReLU gradient, rounded to BF16 for the tensor-core products
-__global__ void k_relu_mask(const float *__restrict__ dy, const bf16 *__restrict__ y, bf16 *__restrict__ dz,
-                            long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    dz[i] = __float2bfloat16_rn(__bfloat162float(y[i]) > 0.0f ? dy[i] : 0.0f);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kEw / 32; w++) s += red[w];
+    atomicAdd(loss, s);
+  }
 }
 
 // wt[ci][tap][co] = w[co][8 - tap][ci]: the data gradient as a forward conv
@@ -810,10 +876,12 @@ __global__ void k_to_bf16(const float *__restrict__ a, bf16 *__restrict__ b, lon
 }
 
 // Interior statistics, per block: part[block][0..3] = sum a^2, sum b,
-// sum b^2, max c (c >= 0); k_stats_final adds the blocks in order.
+// sum b^2, max c (c >= 0); the block that ends last adds them in block order
+// into s[0..3], one thread a sum (a launch of its own, one thread for all of
+// them, took 41 us), and leaves `done` at zero.
 __global__ void k_stats(const float *__restrict__ a, const float *__restrict__ b,
                         const float *__restrict__ c, int nzpad, int x0, int z0, int nx, int nz,
-                        double *__restrict__ part) {
+                        double *__restrict__ part, double *__restrict__ s, unsigned *__restrict__ done) {
   double sa = 0, sb = 0, sb2 = 0, mc = 0;
   const long long total = (long long)nx * nz;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
@@ -831,6 +899,7 @@ __global__ void k_stats(const float *__restrict__ a, const float *__restrict__ b
     mc = fmax(mc, __shfl_down_sync(0xffffffffu, mc, o));
   }
   __shared__ double red[kEw / 32][4];
+  __shared__ bool last;
   if ((threadIdx.x & 31) == 0) {
     red[threadIdx.x >> 5][0] = sa;
     red[threadIdx.x >> 5][1] = sb;
@@ -850,21 +919,24 @@ __global__ void k_stats(const float *__restrict__ a, const float *__restrict__ b
     part[4 * blockIdx.x + 1] = t1;
     part[4 * blockIdx.x + 2] = t2;
     part[4 * blockIdx.x + 3] = t3;
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
   }
-}
-
-__global__ void k_stats_final(const double *__restrict__ part, int blocks, double *__restrict__ s) {
-  double t0 = 0, t1 = 0, t2 = 0, t3 = 0;
-  for (int i = 0; i < blocks; i++) {
-    t0 += part[4 * i];
-    t1 += part[4 * i + 1];
-    t2 += part[4 * i + 2];
-    t3 = fmax(t3, part[4 * i + 3]);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  __shared__ double all[4 * kEw];
+  for (int i = threadIdx.x; i < 4 * kEw; i += kEw) all[i] = i < 4 * (int)gridDim.x ? __ldcg(part + i) : 0.0;
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double t = 0;
+    for (int i = 0; i < (int)gridDim.x; i++) {
+      const double v = all[4 * i + threadIdx.x];
+      t = threadIdx.x == 3 ? fmax(t, v) : t + v;
+    }
+    s[threadIdx.x] = t;
   }
-  s[0] = t0;
-  s[1] = t1;
-  s[2] = t2;
-  s[3] = t3;
+  if (threadIdx.x == 0) *done = 0;
 }
 
 __global__ void k_features(const float *__restrict__ gr, const float *__restrict__ vel,
@@ -906,13 +978,14 @@ __global__ void k_target(const float *__restrict__ dv, int nzpad, int x0, int z0
   }
 }
 
-__global__ void k_scatter(const float *__restrict__ y, int nzpad, int x0, int z0, int nx, int nz,
+// the whole padded grid: y in the interior, zeros around it
+__global__ void k_scatter(const float *__restrict__ y, int nxpad, int nzpad, int x0, int z0, int nx, int nz,
                           int Wp, float *__restrict__ dir) {
-  const long long total = (long long)nx * nz;
+  const long long total = (long long)nxpad * nzpad;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
-    const int ix = (int)(e / nz), iz = (int)(e - (long long)ix * nz);
-    dir[(long long)(x0 + ix) * nzpad + z0 + iz] = y[(long long)ix * Wp + iz];
+    const int x = (int)(e / nzpad), ix = x - x0, iz = (int)(e - (long long)x * nzpad) - z0;
+    dir[e] = ix >= 0 && ix < nx && iz >= 0 && iz < nz ? y[(long long)ix * Wp + iz] : 0.0f;
   }
 }
 
@@ -962,6 +1035,12 @@ void conv_tc_go(const bf16 *in, int cin, const bf16 *w, const float *bias, void 
 
 constexpr int kRedBlocks = 256;           // blocks of the channel sums
 
+void reduce_rows(const RowSum &a, const RowSum &b, cudaStream_t st) {
+  const unsigned na = (unsigned)((a.len + 31) / 32), nb = b.rows ? (unsigned)((b.len + 31) / 32) : 0;
+  k_reduce_rows<<<na + nb, kEw, 0, st>>>(a, b, na);
+  noted();
+}
+
 // Pixels per chunk of a weight gradient: a multiple of one round (64), about
 // 444 CTAs (3 per SM) over the column tiles.
 long long wgrad_pix_per_chunk(long long P, int cin) {
@@ -990,8 +1069,9 @@ void wgrad_tc_cin(const bf16 *dz, int cout, const bf16 *x, float *part, int N, i
   k_wgrad_tc<CIN><<<grid, 128, wgrad_tc_smem(CIN), st>>>(dz, cout, x, part, N, H, W, (int)ppc);
 }
 
-void wgrad_tc_go(const bf16 *dz, int cout, const bf16 *x, int cin, float *dw, float *part, int N, int H, int W,
-                 cudaStream_t st) {
+// bias: partials of the bias gradient to sum in the same launch (rows 0: none)
+void wgrad_tc_go(const bf16 *dz, int cout, const bf16 *x, int cin, float *dw, float *part, const RowSum &bias, int N,
+                 int H, int W, cudaStream_t st) {
   const long long P = (long long)N * H * W;
   const long long ppc = wgrad_pix_per_chunk(P, cin);
   const unsigned chunks = (unsigned)((P + ppc - 1) / ppc);
@@ -1005,20 +1085,23 @@ void wgrad_tc_go(const bf16 *dz, int cout, const bf16 *x, int cin, float *dw, fl
     default: throw Error(SWFWI_ERR_BAD_ARG, "weight gradient: input width must be 16/32/48/64/96/128");
   }
   noted();
-  const long long len = (long long)cout * 9 * cin;
-  k_reduce_rows<<<blocks_for(len), kEw, 0, st>>>(part, (int)chunks, len, dw);
-  noted();
+  reduce_rows({part, (int)chunks, (long long)cout * 9 * cin, dw}, bias, st);
 }
 
-// Channel sums into out[C] (overwritten), in a fixed order.
-void chan_sum(const bf16 *a, const float *wgt, long long P, int C, float *out, float *part, cudaStream_t st) {
-  k_chan_dot<<<kRedBlocks, kEw, 0, st>>>(a, wgt, P, C, part);
+// Partial channel sums of a (times wgt, if given) for out[C], in a fixed order.
+RowSum chan_sum(const bf16 *a, const float *wgt, long long P, int C, float *out, float *part, cudaStream_t st) {
+  if (wgt) k_chan_dot<true><<<kRedBlocks, kDotThreads, 0, st>>>(a, wgt, P, C, part);
+  else k_chan_dot<false><<<kRedBlocks, kDotThreads, 0, st>>>(a, nullptr, P, C, part);
   noted();
-  k_reduce_rows<<<1, kEw, 0, st>>>(part, kRedBlocks, C, out);
-  noted();
+  return {part, kRedBlocks, C, out};
 }
 
 int roundup8(int v) { return (v + 7) / 8 * 8; }
+
+// grid of the kernels that take an image row a blockIdx.y, 8 of C channels a thread
+dim3 row_grid(int C, int rows, int W) {
+  return dim3((unsigned)((W * (C / 8) + kRowThreads - 1) / kRowThreads), (unsigned)rows);
+}
 
 }  // namespace
 
@@ -1092,7 +1175,7 @@ void launch_conv3x3_wgrad(const bf16 *dz, int cout, const bf16 *x, int cin, floa
                 "weight gradient: input width must be 16/32/48/64/96/128");
   SWFWI_REQUIRE(scratch && scratch_floats >= conv3x3_wgrad_scratch(cout, cin, N, H, W),
                 "weight gradient scratch too small");
-  wgrad_tc_go(dz, cout, x, cin, dw, scratch, N, H, W, st);
+  wgrad_tc_go(dz, cout, x, cin, dw, scratch, RowSum{}, N, H, W, st);
 }
 
 void launch_illum_accum(float *illum, const float *p, long long fstride, int n, int nxpad, int nzpad,
@@ -1136,6 +1219,8 @@ Preconditioner::Preconditioner(const int widths[4]) {
   wbf_.resize(nparam_);
   wflip_.resize(maxw);
   red_.resize(8 + 4 * 256);   // loss, statistics and their per-block partials
+  done_.resize(1);
+  done_.zero(st_);
   // He-uniform conv weights, zero biases, small output layer (seeded)
   std::vector<float> h(nparam_, 0.0f);
   std::mt19937 gen(12345u);
@@ -1223,15 +1308,15 @@ void Preconditioner::forward(const float *x, float *y, int N, int H, int W) {
   noted();
   conv_fwd(6, p2_.get(), a3_.get(), P3, H3, W3);
   conv_fwd(7, a3_.get(), b3_.get(), P3, H3, W3);
-  k_upcat<<<blocks_for(P2 * (c3 + c2) / 2), kEw, 0, st_>>>(b3_.get(), c3, s2_.get(), c2, cat2_.get(), N, H2, W2);
+  k_upcat<<<row_grid(c3 + c2, N * H2, W2), kRowThreads, 0, st_>>>(b3_.get(), c3, s2_.get(), c2, cat2_.get(), H2, W2);
   noted();
   conv_fwd(8, cat2_.get(), a4_.get(), P2, H2, W2);
   conv_fwd(9, a4_.get(), u2_.get(), P2, H2, W2);
-  k_upcat<<<blocks_for(P1 * (c2 + c1) / 2), kEw, 0, st_>>>(u2_.get(), c2, s1_.get(), c1, cat1_.get(), N, H1, W1);
+  k_upcat<<<row_grid(c2 + c1, N * H1, W1), kRowThreads, 0, st_>>>(u2_.get(), c2, s1_.get(), c1, cat1_.get(), H1, W1);
   noted();
   conv_fwd(10, cat1_.get(), a5_.get(), P1, H1, W1);
   conv_fwd(11, a5_.get(), u1_.get(), P1, H1, W1);
-  k_upcat<<<blocks_for(P0 * (c1 + c0) / 2), kEw, 0, st_>>>(u1_.get(), c1, s0_.get(), c0, cat0_.get(), N, H, W);
+  k_upcat<<<row_grid(c1 + c0, N * H, W), kRowThreads, 0, st_>>>(u1_.get(), c1, s0_.get(), c0, cat0_.get(), H, W);
   noted();
   conv_fwd(12, cat0_.get(), a6_.get(), P0, H, W);
   conv_fwd(13, a6_.get(), u0_.get(), P0, H, W);
@@ -1241,15 +1326,15 @@ void Preconditioner::forward(const float *x, float *y, int N, int H, int W) {
   if (y) SWFWI_CUDA(cudaMemcpyAsync(y, y_.get(), sizeof(float) * P0, cudaMemcpyDeviceToDevice, st_));
 }
 
-void Preconditioner::conv_bwd(int l, const bf16 *in, const bf16 *out, const float *dY, float *dX,
-                              int H, int W) {
+template <int MODE>
+void Preconditioner::conv_bwd(int l, const bf16 *in, const bf16 *out, const float *a, const float *b, int Ct, int C1,
+                              float *dX, int H, int W) {
   const ConvSpec &s = conv_[l];
   const long long P = (long long)N_ * H * W;
-  k_relu_mask<<<blocks_for(P * s.cout), kEw, 0, st_>>>(dY, out, dz_.get(), P * s.cout);
+  k_relu_mask<MODE><<<row_grid(s.cout, N_ * H, W), kRowThreads, 0, st_>>>(a, b, Ct, C1, out, dz_.get(), H, W, s.cout);
   noted();
-  chan_sum(dz_.get(), nullptr, P, s.cout, grads_.get() + s.b_off, part_.get(), st_);
-  launch_conv3x3_wgrad(dz_.get(), s.cout, in, s.cin, grads_.get() + s.w_off, part_.get(), part_.size(), N_, H, W,
-                       st_);
+  const RowSum bias = chan_sum(dz_.get(), nullptr, P, s.cout, grads_.get() + s.b_off, bpart_.get(), st_);
+  wgrad_tc_go(dz_.get(), s.cout, in, s.cin, grads_.get() + s.w_off, part_.get(), bias, N_, H, W, st_);
   if (dX) {
     k_flip<<<blocks_for((long long)s.cout * 9 * s.cin), kEw, 0, st_>>>(wbf_.get() + s.w_off, wflip_.get(),
                                                                         s.cout, s.cin);
@@ -1264,17 +1349,15 @@ double Preconditioner::backward(const float *t) {
   const int c0 = w_[0], c1 = w_[1], c2 = w_[2], c3 = w_[3];
   const long long P0 = (long long)N * H * W, P1 = P0 / 4, P2 = P0 / 16, P3 = P0 / 64;
   const int H1 = H / 2, W1 = W / 2, H2 = H / 4, W2 = W / 4, H3 = H / 8, W3 = W / 8;
-  const long long big = std::max({P0 * (c1 + c0), P1 * (c2 + c1), P2 * (c3 + c2), P0 * c0});
+  const long long big = std::max({P0 * c0, P1 * std::max(c0, c1), P2 * std::max(c1, c2), P3 * std::max(c2, c3)});
   dy_.resize(P0);
   dA_.resize(big);
-  dB_.resize(big);
-  dCat_.resize(big);
-  dLow_.resize(big);
-  dS0_.resize(P0 * c0);
-  dS1_.resize(P1 * c1);
-  dS2_.resize(P2 * c2);
+  dCat0_.resize(P0 * (c1 + c0));
+  dCat1_.resize(P1 * (c2 + c1));
+  dCat2_.resize(P2 * (c3 + c2));
   dz_.resize(big);
-  size_t need = (size_t)kRedBlocks * 64;
+  bpart_.resize((size_t)kRedBlocks * 64);
+  size_t need = kRedBlocks;
   {
     const int hw[4][2] = {{H, W}, {H1, W1}, {H2, W2}, {H3, W3}};
     const int level[kConvs] = {0, 0, 1, 1, 2, 2, 3, 3, 2, 2, 1, 1, 0, 0};
@@ -1285,55 +1368,38 @@ double Preconditioner::backward(const float *t) {
   part_.resize(need);
   grads_.zero(st_);
   red_.zero(st_);
-  k_mse<<<blocks_for(P0), kEw, 0, st_>>>(y_.get(), t, dy_.get(), P0, 2.0f / (float)P0, red_.get());
+  k_mse<<<(unsigned)std::min<long long>(blocks_for(P0), 592), kEw, 0, st_>>>(y_.get(), t, dy_.get(), P0,
+                                                                             2.0f / (float)P0, red_.get());
   noted();
   // output layer
-  chan_sum(u0_.get(), dy_.get(), P0, c0, grads_.get() + out_w_, part_.get(), st_);
   k_sum<<<kRedBlocks, kEw, 0, st_>>>(dy_.get(), P0, part_.get());
   noted();
-  k_reduce_rows<<<1, kEw, 0, st_>>>(part_.get(), kRedBlocks, 1, grads_.get() + out_b_);
-  noted();
-  k_out_bwd_dx<<<blocks_for(P0 * c0), kEw, 0, st_>>>(dy_.get(), params_.get() + out_w_, dA_.get(), P0, c0);
-  noted();
+  reduce_rows({part_.get(), kRedBlocks, 1, grads_.get() + out_b_},
+              chan_sum(u0_.get(), dy_.get(), P0, c0, grads_.get() + out_w_, bpart_.get(), st_), st_);
+  // A layer's output gradient is formed where it is masked (k_relu_mask):
+  // from the output layer, the four copies of an upsampled pixel, a skip's
+  // two shares, or the convolution above.
   // decoder level 0
-  conv_bwd(13, a6_.get(), u0_.get(), dA_.get(), dB_.get(), H, W);
-  conv_bwd(12, cat0_.get(), a6_.get(), dB_.get(), dCat_.get(), H, W);
-  k_upcat_bwd_low<<<blocks_for(P1 * c1), kEw, 0, st_>>>(dCat_.get(), c1 + c0, c1, dLow_.get(), N, H1, W1);
-  noted();
-  k_upcat_bwd_skip<<<blocks_for(P0 * c0), kEw, 0, st_>>>(dCat_.get(), c1 + c0, c1, dS0_.get(), P0, c0);
-  noted();
+  conv_bwd<kOut>(13, a6_.get(), u0_.get(), dy_.get(), params_.get() + out_w_, 0, 0, dA_.get(), H, W);
+  conv_bwd<kPlain>(12, cat0_.get(), a6_.get(), dA_.get(), nullptr, 0, 0, dCat0_.get(), H, W);
   // decoder level 1
-  conv_bwd(11, a5_.get(), u1_.get(), dLow_.get(), dA_.get(), H1, W1);
-  conv_bwd(10, cat1_.get(), a5_.get(), dA_.get(), dCat_.get(), H1, W1);
-  k_upcat_bwd_low<<<blocks_for(P2 * c2), kEw, 0, st_>>>(dCat_.get(), c2 + c1, c2, dLow_.get(), N, H2, W2);
-  noted();
-  k_upcat_bwd_skip<<<blocks_for(P1 * c1), kEw, 0, st_>>>(dCat_.get(), c2 + c1, c2, dS1_.get(), P1, c1);
-  noted();
+  conv_bwd<kLow>(11, a5_.get(), u1_.get(), dCat0_.get(), nullptr, c1 + c0, 0, dA_.get(), H1, W1);
+  conv_bwd<kPlain>(10, cat1_.get(), a5_.get(), dA_.get(), nullptr, 0, 0, dCat1_.get(), H1, W1);
   // decoder level 2
-  conv_bwd(9, a4_.get(), u2_.get(), dLow_.get(), dA_.get(), H2, W2);
-  conv_bwd(8, cat2_.get(), a4_.get(), dA_.get(), dCat_.get(), H2, W2);
-  k_upcat_bwd_low<<<blocks_for(P3 * c3), kEw, 0, st_>>>(dCat_.get(), c3 + c2, c3, dLow_.get(), N, H3, W3);
-  noted();
-  k_upcat_bwd_skip<<<blocks_for(P2 * c2), kEw, 0, st_>>>(dCat_.get(), c3 + c2, c3, dS2_.get(), P2, c2);
-  noted();
+  conv_bwd<kLow>(9, a4_.get(), u2_.get(), dCat1_.get(), nullptr, c2 + c1, 0, dA_.get(), H2, W2);
+  conv_bwd<kPlain>(8, cat2_.get(), a4_.get(), dA_.get(), nullptr, 0, 0, dCat2_.get(), H2, W2);
   // bottleneck
-  conv_bwd(7, a3_.get(), b3_.get(), dLow_.get(), dA_.get(), H3, W3);
-  conv_bwd(6, p2_.get(), a3_.get(), dA_.get(), dB_.get(), H3, W3);
-  k_pool_bwd<<<blocks_for(P2 * c2), kEw, 0, st_>>>(dB_.get(), dS2_.get(), N, H2, W2, c2);
-  noted();
+  conv_bwd<kLow>(7, a3_.get(), b3_.get(), dCat2_.get(), nullptr, c3 + c2, 0, dA_.get(), H3, W3);
+  conv_bwd<kPlain>(6, p2_.get(), a3_.get(), dA_.get(), nullptr, 0, 0, dA_.get(), H3, W3);
   // encoder level 2
-  conv_bwd(5, a2_.get(), s2_.get(), dS2_.get(), dA_.get(), H2, W2);
-  conv_bwd(4, p1_.get(), a2_.get(), dA_.get(), dB_.get(), H2, W2);
-  k_pool_bwd<<<blocks_for(P1 * c1), kEw, 0, st_>>>(dB_.get(), dS1_.get(), N, H1, W1, c1);
-  noted();
+  conv_bwd<kSkip>(5, a2_.get(), s2_.get(), dCat2_.get(), dA_.get(), c3 + c2, c3, dA_.get(), H2, W2);
+  conv_bwd<kPlain>(4, p1_.get(), a2_.get(), dA_.get(), nullptr, 0, 0, dA_.get(), H2, W2);
   // encoder level 1
-  conv_bwd(3, a1_.get(), s1_.get(), dS1_.get(), dA_.get(), H1, W1);
-  conv_bwd(2, p0_.get(), a1_.get(), dA_.get(), dB_.get(), H1, W1);
-  k_pool_bwd<<<blocks_for(P0 * c0), kEw, 0, st_>>>(dB_.get(), dS0_.get(), N, H, W, c0);
-  noted();
+  conv_bwd<kSkip>(3, a1_.get(), s1_.get(), dCat1_.get(), dA_.get(), c2 + c1, c2, dA_.get(), H1, W1);
+  conv_bwd<kPlain>(2, p0_.get(), a1_.get(), dA_.get(), nullptr, 0, 0, dA_.get(), H1, W1);
   // encoder level 0
-  conv_bwd(1, a0_.get(), s0_.get(), dS0_.get(), dA_.get(), H, W);
-  conv_bwd(0, x16_.get(), a0_.get(), dA_.get(), nullptr, H, W);
+  conv_bwd<kSkip>(1, a0_.get(), s0_.get(), dCat0_.get(), dA_.get(), c1 + c0, c1, dA_.get(), H, W);
+  conv_bwd<kPlain>(0, x16_.get(), a0_.get(), dA_.get(), nullptr, 0, 0, nullptr, H, W);
   double loss = 0;
   SWFWI_CUDA(cudaMemcpyAsync(&loss, red_.get(), sizeof(double), cudaMemcpyDeviceToHost, st_));
   SWFWI_CUDA(cudaStreamSynchronize(st_));
@@ -1370,9 +1436,8 @@ void Preconditioner::stats(const float *a, const float *b, const float *c, int n
                            int nz) {
   constexpr int blocks = 256;
   red_.resize(8 + 4 * blocks);
-  k_stats<<<blocks, kEw, 0, st_>>>(a, b, c, nzpad, x0, z0, nx, nz, red_.get() + 8);
-  noted();
-  k_stats_final<<<1, 1, 0, st_>>>(red_.get() + 8, blocks, red_.get());
+  static_assert(blocks <= kEw, "k_stats sums at most kEw blocks");
+  k_stats<<<blocks, kEw, 0, st_>>>(a, b, c, nzpad, x0, z0, nx, nz, red_.get() + 8, red_.get(), done_.get());
   noted();
 }
 
@@ -1404,8 +1469,8 @@ void Preconditioner::scatter(const float *y, int nxpad, int nzpad, int bx0, int 
   SWFWI_REQUIRE(y && dir, "null field");
   const int nx = nxpad - bx0 - bxn, nz = nzpad - bz0 - bzn;
   SWFWI_REQUIRE(nx > 0 && nz > 0, "empty interior");
-  SWFWI_CUDA(cudaMemsetAsync(dir, 0, sizeof(float) * (size_t)nxpad * nzpad, st_));
-  k_scatter<<<blocks_for((long long)nx * nz), kEw, 0, st_>>>(y, nzpad, bx0, bz0, nx, nz, roundup8(nz), dir);
+  k_scatter<<<blocks_for((long long)nxpad * nzpad), kEw, 0, st_>>>(y, nxpad, nzpad, bx0, bz0, nx, nz, roundup8(nz),
+                                                                    dir);
   noted();
 }
 

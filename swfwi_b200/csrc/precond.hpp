@@ -93,19 +93,22 @@ class Preconditioner {
       cat1_, a5_, u1_, cat0_, a6_, u0_;
   DevBuf<float> y_;
   // backward scratch
-  DevBuf<float> dy_, dA_, dB_, dS0_, dS1_, dS2_, dLow_, dCat_;
+  DevBuf<float> dy_, dA_, dCat0_, dCat1_, dCat2_;
   DevBuf<__nv_bfloat16> dz_;
   DevBuf<float> part_;   // per-chunk / per-block partial sums of the gradients
+  DevBuf<float> bpart_;  // the same of the bias gradients
   DevBuf<double> red_;
+  DevBuf<unsigned> done_;   // blocks of a statistics launch that have ended
   DevBuf<float> feat_, outimg_;
 
   void refresh_bf16();
   // interior statistics of a, b, c into red_[0..3] (fixed summation order)
   void stats(const float *a, const float *b, const float *c, int nzpad, int x0, int z0, int nx, int nz);
   void conv_fwd(int l, const __nv_bfloat16 *in, __nv_bfloat16 *out, long long P, int H, int W);
-  // dY (FP32, layer output grad) -> parameter grads; dX (FP32, may be null)
-  void conv_bwd(int l, const __nv_bfloat16 *in, const __nv_bfloat16 *out, const float *dY, float *dX,
-                int H, int W);
+  // a, b (FP32, see k_relu_mask) -> output gradient -> parameter grads; dX (FP32, may be null or a)
+  template <int MODE>
+  void conv_bwd(int l, const __nv_bfloat16 *in, const __nv_bfloat16 *out, const float *a, const float *b, int Ct,
+                int C1, float *dX, int H, int W);
 };
 
 // Device launches used by the class and the tests.
