@@ -421,30 +421,46 @@ __global__ void __launch_bounds__(128) k_conv3x3_tg(const bf16 *__restrict__ in,
 // Both operands are MN-major (NHWC keeps a pixel's channels contiguous), as
 // core matrices without swizzle: 8 pixels x 16 bytes (8 channels), the
 // 8-channel groups 128 B apart, the two 8-pixel halves of a 16-pixel step
-// (16 groups x 128 B) apart.  Rounds of kWgRound steps are copied with
-// cp.async into two stages while the tensor cores run the previous round;
-// each round's MMAs are committed to its stage's mbarrier (bounded waits).
+// all of a pixel's groups apart.  Rows of D past cout come from whatever lies
+// behind A and are never read.
+// Rounds of kWgRound steps go through a ring of stages: two groups of 128
+// threads copy alternate rounds with cp.async (a thread one 8-channel half
+// of every 16 of a pixel: the pixel's place in the image and its border tests
+// once a round, no divisions) and arrive on the stage's `full` barrier when
+// their copies have landed, a ninth warp issues the round's MMAs and commits
+// them to its `empty` barrier; nothing else synchronises, and all waits are
+// bounded.  The copies bound it: 1.2 million pixels take 113 us for 16 -> 16
+// channels and 374 for 48 -> 16; 222 and 645 with one group, two stages, a
+// CTA barrier a round and zeros copied into A's groups past cout.
 // The chunks are summed afterwards in a fixed order (k_reduce_rows):
 // training stays bit-reproducible.
 constexpr int kWgRound = 4;   // 16-pixel steps per round (64 pixels)
+constexpr int kWgThreads = 288;
 
 __host__ __device__ inline int wg_tiles(int cin) { return (9 * cin + 255) / 256; }
 __host__ __device__ inline int wg_cols(int cin) { return ((9 * cin + wg_tiles(cin) - 1) / wg_tiles(cin) + 15) / 16 * 16; }
-__host__ __device__ inline int wg_stage_bytes(int cin) { return kWgRound * (4096 + 32 * wg_cols(cin)); }
+__host__ __device__ inline int wg_stage_bytes(int cin, int cout) { return kWgRound * 32 * (cout + wg_cols(cin)); }
+// stages: four if two CTAs then fit an SM (their accumulators take half of
+// the tensor memory each), or three, or four for one CTA
+__host__ __device__ inline int wg_stages(int cin, int cout) {
+  const int sb = wg_stage_bytes(cin, cout), two = 112 * 1024;
+  return 4 * sb <= two ? 4 : 3 * sb <= two ? 3 : 4;
+}
 
-// CIN is a template parameter: the staging divides by constants.
+// CIN is a template parameter: the copies' loops are by constants.
 template <int CIN>
-__global__ void __launch_bounds__(128) k_wgrad_tc(const bf16 *__restrict__ dz, int cout, const bf16 *__restrict__ x,
-                                                  float *__restrict__ part, int N, int H, int W, int ppc) {
+__global__ void __launch_bounds__(kWgThreads) k_wgrad_tc(const bf16 *__restrict__ dz, int cout,
+                                                         const bf16 *__restrict__ x, float *__restrict__ part, int N,
+                                                         int H, int W, int ppc) {
   using namespace stream_detail;
   extern __shared__ __align__(1024) unsigned char sm[];
   constexpr int cin = CIN;
   const int NT = 9 * cin, NNmax = wg_cols(cin);
   const int n0 = blockIdx.y * NNmax, NN = min(NNmax, NT - n0);   // this CTA's columns
-  const int SB = wg_stage_bytes(cin);
-  uint64_t *bar = reinterpret_cast<uint64_t *>(sm + 2 * SB);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 2);
-  int *dec = reinterpret_cast<int *>(bar + 3);   // [stage][3][64]: n (-1: none), h, w of the round's pixels
+  const int SB = wg_stage_bytes(cin, cout), S = wg_stages(cin, cout);
+  uint64_t *full = reinterpret_cast<uint64_t *>(sm + S * SB), *empty = full + 4, *done = empty + 4;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
+  volatile int *bad = reinterpret_cast<volatile int *>(tslot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long HW = (long long)H * W, P = (long long)N * HW;
   const long long pb = (long long)blockIdx.x * ppc, pe = min(P, pb + ppc);
@@ -457,78 +473,116 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const bf16 *__restrict__ dz, i
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+    for (int k = 0; k < 4; k++) {
+      mbar_init(&full[k], 128);
+      mbar_init(&empty[k], 1);
+    }
+    mbar_init(done, 1);
+    *bad = 0;
     fence_mbar_init();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t taddr = *tslot;
-  // kind::f16: FP32 accumulator, BF16 A and B, both MN-major, N = NN, M = 128
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
-                         ((uint32_t)(NN >> 3) << 17) | ((128u >> 4) << 24);
   const uint32_t sbase = tc::saddr(sm);
-  const int zgroups = cout / 8, bgroups = NN / 8;
 
-  auto load_round = [&](int rd) {
-    const int st = rd & 1;
-    int *dn = dec + st * 192, *dh = dn + 64, *dw = dh + 64;
-    if (tid < 64) {   // decode the round's 64 pixels once
-      const long long p = pb + (long long)rd * 64 + tid;
-      const int n = p < pe ? (int)(p / HW) : -1;
-      const int r = p < pe ? (int)(p - (long long)n * HW) : 0;
-      dn[tid] = n;
-      dh[tid] = r / W;
-      dw[tid] = r - (r / W) * W;
-    }
-    __syncthreads();
-    const uint32_t sa = sbase + (uint32_t)(st * SB), sb = sa + (uint32_t)(kWgRound * 4096);
-    // A: 64 pixels x 16 channel groups (groups past cout are zero rows)
-    for (int u = tid; u < 64 * 16; u += 128) {
-      const int g = u & 15, pi = u >> 4, ks = pi >> 4, r = pi & 15;
-      const bool ok = g < zgroups && dn[pi] >= 0;
-      const long long p = pb + (long long)rd * 64 + pi;
-      tc::cp16(sa + (uint32_t)(ks * 4096 + (r >> 3) * 2048 + g * 128 + (r & 7) * 16), ok ? dz + p * cout + g * 8 : dz,
-               ok);
-    }
-    // B: 64 pixels x this tile's (tap, 8-channel) groups, zero outside the image
-    for (int u = tid; u < 64 * bgroups; u += 128) {
-      const int g = u % bgroups, pi = u / bgroups, ks = pi >> 4, r = pi & 15;
-      const int col = n0 + g * 8, tap = col / cin, c8 = col - tap * cin;
-      const int ky = tap / 3, kx = tap - 3 * ky;
-      const int n = dn[pi], hh = dh[pi] + ky - 1, xx = dw[pi] + kx - 1;
-      const bool ok = n >= 0 && hh >= 0 && hh < H && xx >= 0 && xx < W;
-      tc::cp16(sb + (uint32_t)(ks * NN * 32 + (r >> 3) * (NN * 16) + g * 128 + (r & 7) * 16),
-               ok ? x + (((long long)n * H + hh) * W + xx) * cin + c8 : x, ok);
-    }
-    tc::cp_commit();
-  };
-
-  bool ok = true;
-  if (R > 0) load_round(0);
-  for (int rd = 0; rd < R && ok; rd++) {
-    if (rd + 1 < R) {
-      if (rd >= 1 && !__syncthreads_and(mbar_wait(&bar[(rd + 1) & 1], (uint32_t)(((rd - 1) >> 1) & 1)))) {
-        ok = false;
+  if (warp < 8) {
+    // ---- copies: pixel pi of the rounds rd = warp / 4, + 2, ..., channels
+    // 8 * half .. of every 16
+    const int half = tid & 1, pi = (tid >> 1) & 63, ks = pi >> 4, r = pi & 15;
+    const uint32_t da = (uint32_t)(ks * 32 * cout + (r >> 3) * 16 * cout + half * 128 + (r & 7) * 16);
+    const uint32_t db = (uint32_t)(kWgRound * 32 * cout + ks * 32 * NN + (r >> 3) * 16 * NN + half * 128 + (r & 7) * 16);
+    int rd = warp >> 2;
+    long long p = pb + (long long)rd * 64 + pi;
+    int h = (int)((p % HW) / W), w = (int)(p % W);
+    const int tap0 = n0 / cin, c0 = n0 - tap0 * cin + 8 * half;
+    auto landed = [&](int round) {
+      // written through the generic proxy, read by the MMAs through the async proxy
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::saddr(&full[round % S])) : "memory");
+    };
+    int last = -1;   // this group's round that has been copied but not announced
+    for (; rd < R; rd += 2) {
+      const int st = rd % S;
+      if (*bad) break;
+      if (rd >= S && !mbar_wait(&empty[st], (uint32_t)((rd / S - 1) & 1))) {
+        *bad = 1;
         break;
       }
-      load_round(rd + 1);
-      tc::cp_wait<1>();
-    } else {
-      tc::cp_wait<0>();
+      const uint32_t stage = sbase + (uint32_t)(st * SB);
+      const bool in = p < pe;
+      const bf16 *za = in ? dz + p * cout + 8 * half : dz;
+      for (int g = 0; g < cout; g += 16) tc::cp16(stage + da + (uint32_t)(g * 16), in ? za + g : dz, in);
+      // bit 3 * ky + kx: the tap's pixel is inside the image
+      unsigned rows = (h > 0 ? 1u : 0u) | 2u | (h + 1 < H ? 4u : 0u);
+      const unsigned cols = (w > 0 ? 1u : 0u) | 2u | (w + 1 < W ? 4u : 0u);
+      unsigned vm = ((rows & 1u) ? cols : 0u) | ((rows & 2u) ? cols << 3 : 0u) | ((rows & 4u) ? cols << 6 : 0u);
+      if (!in) vm = 0u;
+      const bf16 *xp = x + p * cin;
+      if constexpr (9 * CIN <= 256) {
+#pragma unroll
+        for (int tap = 0; tap < 9; tap++) {
+          const bool ok = vm >> tap & 1u;
+          const bf16 *src = xp + ((tap / 3 - 1) * W + tap % 3 - 1) * cin + 8 * half;
+#pragma unroll
+          for (int c = 0; c < cin; c += 16)
+            tc::cp16(stage + db + (uint32_t)((tap * cin + c) * 16), ok ? src + c : x, ok);
+        }
+      } else {
+        int tap = tap0, c = c0, kx = tap0 % 3;
+        const bf16 *src = xp + ((tap0 / 3 - 1) * W + kx - 1) * cin;
+#pragma unroll 2
+        for (int g = 0; g < NN; g += 16) {
+          const bool ok = vm >> tap & 1u;
+          tc::cp16(stage + db + (uint32_t)(g * 16), ok ? src + c : x, ok);
+          c += 16;
+          if (c >= cin) {
+            c -= cin;
+            tap++;
+            kx++;
+            src += cin;
+            if (kx == 3) {
+              kx = 0;
+              src += (W - 3) * cin;
+            }
+          }
+        }
+      }
+      tc::cp_commit();
+      if (last >= 0) {
+        tc::cp_wait<1>();
+        landed(last);
+      }
+      last = rd;
+      p += 128;
+      w += 128;
+      while (w >= W) {
+        w -= W;
+        if (++h == H) h = 0;
+      }
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
+    tc::cp_wait<0>();
+    if (last >= 0) landed(last);
+  } else if (lane == 0) {
+    // ---- MMAs.  kind::f16: FP32 accumulator, BF16 A and B, both MN-major, N = NN, M = 128
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                           ((uint32_t)(NN >> 3) << 17) | ((128u >> 4) << 24);
+    for (int rd = 0; rd < R; rd++) {
+      const int st = rd % S;
+      if (*bad) break;
+      if (!mbar_wait(&full[st], (uint32_t)((rd / S) & 1))) {
+        *bad = 1;
+        break;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t sa = sbase + (uint32_t)((rd & 1) * SB), sb = sa + (uint32_t)(kWgRound * 4096);
+      const uint32_t sa = sbase + (uint32_t)(st * SB), sb = sa + (uint32_t)(kWgRound * 32 * cout);
       for (int ks = 0; ks < kWgRound; ks++) {
         // MN-major descriptors: leading (K-half) offset, stride (8-channel group) offset 128
-        const uint64_t ad = (uint64_t)(((sa + ks * 4096) >> 4) & 0x3FFFu) | ((uint64_t)(2048u >> 4) << 16) |
+        const uint64_t ad = (uint64_t)(((sa + ks * 32 * cout) >> 4) & 0x3FFFu) | ((uint64_t)(uint32_t)cout << 16) |
                             ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
-        const uint64_t bd = (uint64_t)(((sb + ks * NN * 32) >> 4) & 0x3FFFu) |
-                            ((uint64_t)((uint32_t)(NN * 16) >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
+        const uint64_t bd = (uint64_t)(((sb + ks * NN * 32) >> 4) & 0x3FFFu) | ((uint64_t)(uint32_t)NN << 16) |
+                            ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
         const uint32_t acc = (rd > 0 || ks > 0) ? 1u : 0u;
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -537,14 +591,19 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const bf16 *__restrict__ dz, i
             : "memory");
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       tc::saddr(&bar[rd & 1]))
+                       tc::saddr(&empty[st]))
                    : "memory");
     }
+    // whatever has been issued
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc::saddr(done))
+                 : "memory");
   }
-  if (ok && R > 0 && !__syncthreads_and(mbar_wait(&bar[(R - 1) & 1], (uint32_t)(((R - 1) >> 1) & 1)))) ok = false;
-  tc::cp_wait<0>();
+  __syncwarp();
+  if (!mbar_wait(done, 0u)) *bad = 1;
+  __syncthreads();
+  const bool ok = *bad == 0;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (ok && warp * 32 < cout) {   // lanes = output channels
+  if (ok && warp < 4 && warp * 32 < cout) {   // lanes = output channels
     const int co = warp * 32 + lane;
     float *dst = part + ((long long)blockIdx.x * cout + co) * NT + n0;
     for (int c0 = 0; c0 < NN; c0 += 16) {
@@ -570,8 +629,6 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const bf16 *__restrict__ dz, i
     }
   } else if (!ok && tid == 0) {
     atomicExch(&g_conv_timeout, 1);
-    mbar_wait(&bar[0], 0u);   // bounded: whatever MMAs are still in flight
-    mbar_wait(&bar[1], 1u);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1048,10 +1105,9 @@ long long wgrad_pix_per_chunk(long long P, int cin) {
   return 64 * std::max(1LL, (P + 64 * chunks - 1) / (64 * chunks));
 }
 
-size_t wgrad_tc_smem(int cin) {
-  const size_t need = 2 * (size_t)wg_stage_bytes(cin) + 32 + 2 * 3 * 64 * 4;
+size_t wgrad_tc_smem(int cin, int cout) {
+  const size_t need = (size_t)wg_stages(cin, cout) * wg_stage_bytes(cin, cout) + 9 * 8 + 8;
   const int fit = 512 / tc::tmem_cols(wg_cols(cin));   // CTAs whose accumulators fit
-  if (fit >= 16) return need;
   const size_t cap = 228 * 1024 / (fit + 1) - 1024 + 16;   // fit + 1 CTAs no longer fit
   return std::max(need, cap);
 }
@@ -1061,12 +1117,12 @@ void wgrad_tc_cin(const bf16 *dz, int cout, const bf16 *x, float *part, int N, i
                   unsigned chunks, cudaStream_t st) {
   static const bool attr = [] {
     SWFWI_CUDA(cudaFuncSetAttribute(k_wgrad_tc<CIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)wgrad_tc_smem(CIN)));
+                                    227 * 1024));
     return true;
   }();
   (void)attr;
   dim3 grid(chunks, wg_tiles(CIN));
-  k_wgrad_tc<CIN><<<grid, 128, wgrad_tc_smem(CIN), st>>>(dz, cout, x, part, N, H, W, (int)ppc);
+  k_wgrad_tc<CIN><<<grid, kWgThreads, wgrad_tc_smem(CIN, cout), st>>>(dz, cout, x, part, N, H, W, (int)ppc);
 }
 
 // bias: partials of the bias gradient to sum in the same launch (rows 0: none)
