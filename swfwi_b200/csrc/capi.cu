@@ -110,7 +110,7 @@ int swfwi_fd4t10s_damp_zjh_2d_vtrans(float *prev, const float *curr, const float
   return guarded([&] {
     SWFWI_REQUIRE(prev && curr && vel, "null field");
     SWFWI_REQUIRE(nx > 12 && nz > 12 && nb >= 1, "grid too small");
-    launch_step(ARITH_REF, true, false, 32, drop_in_args(prev, curr, vel, nx, nz, nb, 0), 1,
+    launch_step(ARITH_REF, true, false, drop_in_args(prev, curr, vel, nx, nz, nb, 0), 1,
                 as_stream(stream));
     check_launch();
   });
@@ -122,7 +122,7 @@ int swfwi_fd4t10s_zjh_2d_vtrans(float *prev, const float *curr, const float *vel
   return guarded([&] {
     SWFWI_REQUIRE(prev && curr && vel, "null field");
     SWFWI_REQUIRE(nx > 12 && nz > 12, "grid too small");
-    launch_step(ARITH_REF, false, false, 32, drop_in_args(prev, curr, vel, nx, nz, 1, 0), 1,
+    launch_step(ARITH_REF, false, false, drop_in_args(prev, curr, vel, nx, nz, 1, 0), 1,
                 as_stream(stream));
     check_launch();
   });
@@ -138,7 +138,7 @@ int swfwi_fd4t10s_step_batch(float *prev, const float *curr, const float *vel, i
     SWFWI_REQUIRE(nshots == 1 || shot_stride >= (long long)nx * nz, "shot stride too small");
     StepArgs a = drop_in_args(prev, curr, vel, nx, nz, nb, shot_stride);
     a.shots_per_vel = nshots;
-    launch_step(arith, damped != 0, false, 32, a, nshots, as_stream(stream));
+    launch_step(arith, damped != 0, false, a, nshots, as_stream(stream));
     check_launch();
   });
 }
@@ -159,7 +159,7 @@ int swfwi_fd4t10s_step_f64(double *prev, const double *curr, const double *vel, 
     a.shot_stride = 0;
     a.vel_stride = 0;
     a.shots_per_vel = 1;
-    launch_step(ARITH_F64, damped != 0, false, 32, a, 1, as_stream(stream));
+    launch_step(ARITH_F64, damped != 0, false, a, 1, as_stream(stream));
     check_launch();
   });
 }

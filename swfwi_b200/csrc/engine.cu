@@ -469,7 +469,7 @@ void Propagator::step_fields(int ar, bool damped, void *prev, const void *curr, 
     a.shot_stride = fstride;
     a.vel_stride = 0;
     a.shots_per_vel = std::max(n, 1);
-    launch_step(ARITH_F64, damped, true, 32, a, n, st_);
+    launch_step(ARITH_F64, damped, true, a, n, st_);
     step_timer().close(done, st_);
     return;
   }
@@ -530,14 +530,14 @@ StepArgs caller_args(float *p0, const float *p1, const float *vel, int nxpad, in
 void Propagator::step_forward(float *p0, float *p1) {
   SWFWI_REQUIRE(p0 && p1 && vel_, "null field or no velocity");
   cudaEvent_t done = step_timer().open(st_, (double)(nxpad - 12) * (nzpad - 12), 1, 1, 4);
-  launch_step(arith, true, false, 32, caller_args(p0, p1, vel_, nxpad, nzpad, bx0), 1, st_);
+  launch_step(arith, true, false, caller_args(p0, p1, vel_, nxpad, nzpad, bx0), 1, st_);
   step_timer().close(done, st_);
 }
 
 void Propagator::step_backward(float *p0, float *p1) {
   SWFWI_REQUIRE(p0 && p1 && vel_, "null field or no velocity");
   cudaEvent_t done = step_timer().open(st_, (double)(nxpad - 12) * (nzpad - 12), 1, 1, 4);
-  launch_step(arith, false, false, 32, caller_args(p0, p1, vel_, nxpad, nzpad, bx0), 1, st_);
+  launch_step(arith, false, false, caller_args(p0, p1, vel_, nxpad, nzpad, bx0), 1, st_);
   step_timer().close(done, st_);
 }
 

@@ -362,36 +362,53 @@ void launch_image(T *image, long long image_stride, const T *s, const T *r, long
 }
 
 // ---------------------------------------------------------------- step
-template <int ARITH, bool DAMPED, bool RCP, int TX>
+template <int ARITH, bool DAMPED, bool RCP, int TX, int THREADS>
 static void step_t(const StepArgs &a, int nslots, cudaStream_t st) {
-  dim3 g((a.nz - 12 + kTZ - 1) / kTZ, (a.nx - 12 + TX - 1) / TX, nslots);
-  fd_step_tile<ARITH, DAMPED, RCP, TX><<<g, kStepThreads, 0, st>>>(a);
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((a.nz - 12 + kTZ - 1) / kTZ, (a.nx - 12 + TX - 1) / TX, nslots);
+  c.blockDim = dim3(THREADS);
+  c.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  SWFWI_CUDA(cudaLaunchKernelEx(&c, fd_step_tile<ARITH, DAMPED, RCP, TX, THREADS>, a));
   note_launch();
 }
 
+// Tiles of 16 rows and 512 threads while 32-row tiles would be fewer than four
+// an SM: their phases are a quarter of the passes.  Microseconds a launch in
+// a row of them, reference arithmetic, 16 x 512 against 32 x 256: 533 x 193
+// (102 tiles of 32 rows) 4.9 / 6.4, 1000 x 400 (403) 7.2 / 8.4, 1500 x 600
+// (893) 12.7 / 11.4, 3000 x 1000 37 / 29.  (The launch without programmatic
+// serialisation, 32 x 256: 7.2 and 9.5 on the first two.)
+constexpr long long kSmallTiles = 4 * 148;
+
 template <int ARITH, bool DAMPED, bool RCP>
-static void step_tx(int tx, const StepArgs &a, int nslots, cudaStream_t st) {
-  if (tx >= 64) step_t<ARITH, DAMPED, RCP, 64>(a, nslots, st);
-  else step_t<ARITH, DAMPED, RCP, 32>(a, nslots, st);
+static void step_tx(const StepArgs &a, int nslots, cudaStream_t st) {
+  const long long tiles = (long long)((a.nz - 12 + kTZ - 1) / kTZ) * ((a.nx - 12 + 31) / 32) * nslots;
+  if (tiles <= kSmallTiles) step_t<ARITH, DAMPED, RCP, 16, 512>(a, nslots, st);
+  else step_t<ARITH, DAMPED, RCP, 32, 256>(a, nslots, st);
 }
 
 template <int ARITH>
-static void step_a(bool damped, bool rcp, int tx, const StepArgs &a, int nslots, cudaStream_t st) {
+static void step_a(bool damped, bool rcp, const StepArgs &a, int nslots, cudaStream_t st) {
   if (damped) {
-    if (rcp) step_tx<ARITH, true, true>(tx, a, nslots, st);
-    else step_tx<ARITH, true, false>(tx, a, nslots, st);
+    if (rcp) step_tx<ARITH, true, true>(a, nslots, st);
+    else step_tx<ARITH, true, false>(a, nslots, st);
   } else {
-    if (rcp) step_tx<ARITH, false, true>(tx, a, nslots, st);
-    else step_tx<ARITH, false, false>(tx, a, nslots, st);
+    if (rcp) step_tx<ARITH, false, true>(a, nslots, st);
+    else step_tx<ARITH, false, false>(a, nslots, st);
   }
 }
 
-void launch_step(int arith, bool damped, bool vel_is_rcp, int tx, const StepArgs &a, int nslots,
+void launch_step(int arith, bool damped, bool vel_is_rcp, const StepArgs &a, int nslots,
                  cudaStream_t st) {
   if (nslots <= 0 || a.nx <= 12 || a.nz <= 12) return;
-  if (arith == ARITH_REF) step_a<ARITH_REF>(damped, vel_is_rcp, tx, a, nslots, st);
-  else if (arith == ARITH_FAST) step_a<ARITH_FAST>(damped, vel_is_rcp, tx, a, nslots, st);
-  else step_a<ARITH_F64>(damped, vel_is_rcp, tx, a, nslots, st);
+  if (arith == ARITH_REF) step_a<ARITH_REF>(damped, vel_is_rcp, a, nslots, st);
+  else if (arith == ARITH_FAST) step_a<ARITH_FAST>(damped, vel_is_rcp, a, nslots, st);
+  else step_a<ARITH_F64>(damped, vel_is_rcp, a, nslots, st);
 }
 
 // ---------------------------------------------------------------- mute

@@ -107,7 +107,7 @@ void launch_image_sum(float *image, const float *s, const float *r, long long sh
 
 // One FD step for all slots: the shared-memory tile form (any pitch, any
 // arithmetic; stencil.cuh).
-void launch_step(int arith, bool damped, bool vel_is_rcp, int tx, const StepArgs &a, int nslots,
+void launch_step(int arith, bool damped, bool vel_is_rcp, const StepArgs &a, int nslots,
                  cudaStream_t st);
 // Warp-specialised streaming step (stream_ws.cuh): bz = 120, 248 or 376
 // output depths per CTA (1-3 consumer warps), depth = 3 or 7 rows ahead;

@@ -168,17 +168,21 @@ __device__ __forceinline__ float damp_delta(int ix, int iz, int nx, int nz, int 
   return __fmul_rn(__fmul_rn(0.05f, dist), dist);
 }
 
-constexpr int kStepThreads = 256;
+// What bounds a launch on one field is the chain of its phases (fetch, u2,
+// update), each of as many passes as the tile has points a thread; the tile
+// and the threads are the launcher's choice (step_t in kernels.cu).  Launched
+// with programmatic stream serialisation: its blocks are set up while the
+// kernel before it ends, and touch memory once that one's writes are visible.
 constexpr int kTZ = 32;
 
-template <int ARITH, bool DAMPED, bool VEL_IS_RCP, int TX>
-__global__ void __launch_bounds__(kStepThreads)
+template <int ARITH, bool DAMPED, bool VEL_IS_RCP, int TX, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 fd_step_tile(StepArgs a) {
   typedef typename StorageOf<ARITH>::type T;
   constexpr int H = 6;
   constexpr int CX = TX + 2 * H, CZ = kTZ + 2 * H;
   constexpr int UX = TX + 2, UZ = kTZ + 2;
-  constexpr int ROWS = kStepThreads / 32;      // warps, one output row each pass
+  constexpr int ROWS = THREADS / 32;      // warps, one output row each pass
   constexpr int PER = TX / ROWS;               // outputs per thread
   __shared__ T sc[CX * CZ];
   __shared__ T su[UX * UZ];
@@ -195,6 +199,9 @@ fd_step_tile(StepArgs a) {
   const int ty = threadIdx.x >> 5;
   const int gz = z0 + tz;
 
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
   // Early fetch of prev and the velocity term for this thread's outputs.
   T pv[PER], rv[PER];
 #pragma unroll
@@ -210,7 +217,7 @@ fd_step_tile(StepArgs a) {
   }
 
   // Stage the current field with its 6-cell halo.
-  for (int i = threadIdx.x; i < CX * CZ; i += kStepThreads) {
+  for (int i = threadIdx.x; i < CX * CZ; i += THREADS) {
     int lx = i / CZ, lz = i - lx * CZ;
     int gx = x0 - H + lx, gzz = z0 - H + lz;
     T v = 0;
@@ -220,7 +227,7 @@ fd_step_tile(StepArgs a) {
   __syncthreads();
 
   // u2 on the tile plus a one-cell ring.
-  for (int i = threadIdx.x; i < UX * UZ; i += kStepThreads) {
+  for (int i = threadIdx.x; i < UX * UZ; i += THREADS) {
     int ux = i / UZ, uz = i - ux * UZ;
     su[i] = lap10<ARITH, CZ, T>(&sc[(ux + H - 1) * CZ + (uz + H - 1)]);
   }
