@@ -752,7 +752,7 @@ bool Propagator::resident_forward(Work<float> &w, int n, PointSet src, const flo
   if (!resident_allowed()) return false;
   if (save_strips && (recon != SWFWI_RECON_STRIPS || strip_format != SWFWI_STRIP_F32 || illum)) return false;
   const bool geo = rec.pos == d_geo_pos_p_.get();
-  const ResidentPlan p = plan_resident(false, n, nxpad, nzpad, bx0, save_strips, src.per_shot == 1 ? row_src1_ : row_src_,
+  const ResidentPlan p = plan_resident(arith, false, n, nxpad, nzpad, bx0, save_strips, src.per_shot == 1 ? row_src1_ : row_src_,
                                        geo ? row_geo_ : row_rec_);
   if (!resident_faster(p, false, n)) return false;
   if (save_strips) {   // the backward sweep reads the final pair, border zeros included
@@ -803,7 +803,7 @@ bool Propagator::resident_backward(Work<float> &w, int n, PointSet src, const fl
                                    const float *velrcp) {
   if (!resident_allowed()) return false;
   if (recon != SWFWI_RECON_STRIPS || strip_format != SWFWI_STRIP_F32) return false;
-  const ResidentPlan p = plan_resident(true, n, nxpad, nzpad, bx0, true, src.per_shot == 1 ? row_src1_ : row_src_,
+  const ResidentPlan p = plan_resident(arith, true, n, nxpad, nzpad, bx0, true, src.per_shot == 1 ? row_src1_ : row_src_,
                                        rec.pos == d_geo_pos_p_.get() ? row_geo_ : row_rec_);
   if (!resident_faster(p, true, n)) return false;
   int steps = 0;   // the reference's loop images while t > 0.3

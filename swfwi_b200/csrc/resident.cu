@@ -77,34 +77,34 @@ int row_chunks(bool back, int rmax, int ngroups, int warps) {
   return best_k;
 }
 
-template <int ARITH, bool BACK>
+template <int ARITH, bool BACK, bool WIDE>
 void launch_t(const ResidentArgs &a, size_t smem, cudaStream_t st) {
   // raise the dynamic shared memory limit once (thread-safe static init)
-  static const cudaError_t attr = cudaFuncSetAttribute(fd_resident<ARITH, BACK>,
+  static const cudaError_t attr = cudaFuncSetAttribute(fd_resident<ARITH, BACK, WIDE>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
   SWFWI_CUDA(attr);
   ResidentArgs b = a;
   void *args[] = {&b};
-  SWFWI_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fd_resident<ARITH, BACK>),
+  SWFWI_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fd_resident<ARITH, BACK, WIDE>),
                                          dim3(a.nslots * a.cps), dim3(kResidentThreads), args, smem, st));
 }
 
 }  // namespace
 
-ResidentPlan plan_resident(bool back, int n, int nx, int nz, int bx0, bool strips, const std::vector<int> &src_hist,
+static ResidentPlan plan_slabs(bool thin, int arith, bool back, int n, int nx, int nz, int bx0, bool strips, const std::vector<int> &src_hist,
                            const std::vector<int> &rec_hist) {
   ResidentPlan p;
   const int rows = nx - 12;
   if (n <= 0 || rows < 1 || nz < 16) return p;
   const int sms = device_sms(), zp = row_floats(nz);
   if (6LL * depth_groups(nz) * depth_groups(nz) >= (1 << 20)) return p;   // the index divisions by multiplication
-  const int most = std::min(sms, std::max(rows / 6, 1));   // a slab's halo is its neighbours' edge rows
+  const int most = std::min(sms, thin ? rows : std::max(rows / 6, 1));   // a slab's halo: its neighbours' edge rows
   auto smem_of = [&](int cps, int &rmax, int &cs, int &cr, int &cg) {
     rmax = (rows + cps - 1) / cps;
     cs = window_max(src_hist, rmax + 12);
     cr = window_max(rec_hist, rmax + 12);
     cg = back && strips ? stage_cells(nx, nz, bx0, cps) : 0;
-    return resident_smem(back, rmax, zp, cs, cr, cg);
+    return resident_smem(back, false, rmax, zp, cs, cr, cg);
   };
   // fewest slabs whose fields fit beside their lists, from the fewest whose
   // fields fit alone
@@ -122,7 +122,20 @@ ResidentPlan plan_resident(bool back, int n, int nx, int nz, int bx0, bool strip
   p.cps = std::min(most, sms / p.slots);
   p.smem = smem_of(p.cps, p.rmax, p.cap_src, p.cap_rec, p.cap_stage);
   while (p.smem > kMaxSmem && p.cps > cps) p.smem = smem_of(--p.cps, p.rmax, p.cap_src, p.cap_rec, p.cap_stage);
+  p.thin = rows / p.cps < 6;
+  p.rows = rows;
   if (p.smem > kMaxSmem) return ResidentPlan();
+  // The two-pass form: in REF arithmetic wherever it fits, in FAST up to two
+  // rounds of u2 items.  Microseconds a forward step, two-pass / march: REF 1
+  // shot of 533 x 193 2.7 / 4.8, 8 shots 6.0 / 8.3, 16 shots 10.0 / 11.8, 1
+  // shot of 993 x 343 4.4 / 6.0; FAST 1 shot of 533 x 193 (282 items) 2.3 /
+  // 2.9, 4 shots (799) 3.5 / 3.6, 8 shots (1457) 5.1 / 4.4, 1 shot of 993 x
+  // 343 (756) 3.9 / 4.0, 2 shots (1344) 5.0 / 4.6.
+  const long long u2_items = (back ? 2LL : 1LL) * (p.rmax + 2) * depth_groups(nz);
+  const size_t two = resident_smem(back, true, p.rmax, zp, p.cap_src, p.cap_rec, p.cap_stage);
+  p.wide = (arith == ARITH_REF || u2_items <= 800) && two <= kMaxSmem &&
+           u2_items * depth_groups(nz) < (1 << 20);   // the index divisions by multiplication
+  if (p.wide) p.smem = two;
   p.zp = zp;
   p.ngroups = depth_groups(nz);
   p.ogroups = (nz - 7) / 4;
@@ -131,10 +144,19 @@ ResidentPlan plan_resident(bool back, int n, int nx, int nz, int bx0, bool strip
   // 10.6 / 6.2 / 5.5 / 5.5 us a step with 1 / 2 / 3 / 4)
   p.helpers = 3;
   p.chunks = row_chunks(back, p.rmax, p.ngroups, kResidentThreads / 32 - p.helpers);
-  if (resident_halo(p.slots, p.cps, 2, p.ogroups) >= (1u << 31)) return ResidentPlan();
-  p.halo = resident_halo(p.slots, p.cps, back ? 2 : 1, p.ogroups);
+  if (resident_halo(p.slots, p.cps, rows, p.thin, 2, p.ogroups) >= (1u << 31)) return ResidentPlan();
+  p.halo = resident_halo(p.slots, p.cps, rows, p.thin, back ? 2 : 1, p.ogroups);
   p.ok = true;
   return p;
+}
+
+// Slabs of fewer than 6 rows only in the two-pass form, which gains by them
+// (533 x 193, 148 slabs against 86: 1 shot forward, REF, 2.5 / 3.2 us a step;
+// an encoded epoch of 800 steps, FAST, 10.6 / 12.7 ms).
+ResidentPlan plan_resident(int arith, bool back, int n, int nx, int nz, int bx0, bool strips,
+                           const std::vector<int> &src_hist, const std::vector<int> &rec_hist) {
+  const ResidentPlan p = plan_slabs(true, arith, back, n, nx, nz, bx0, strips, src_hist, rec_hist);
+  return p.thin && !p.wide ? plan_slabs(false, arith, back, n, nx, nz, bx0, strips, src_hist, rec_hist) : p;
 }
 
 // Estimated microseconds a step (B200, fits to timed sweeps of 1..96 shots of
@@ -149,8 +171,13 @@ ResidentPlan plan_resident(bool back, int n, int nx, int nz, int bx0, bool strip
 double resident_us(const ResidentPlan &p, int arith, bool back) {
   const double x = (double)p.rmax * p.ngroups;
   const bool ref = arith == ARITH_REF;
-  const double round = back ? (ref ? 3.5 + 0.0066 * x : 2.9 + 0.0028 * x) + 0.045 * p.ogroups
-                            : (ref ? 3.9 + 0.0027 * x : 2.7 + 0.00113 * x);
+  double round;
+  if (p.wide)
+    round = back ? (ref ? 1.5 + 0.0066 * x : 1.7 + 0.0028 * x) + 0.045 * p.ogroups
+                 : (ref ? 2.4 + 0.0028 * x : 2.1 + 0.0021 * x);
+  else
+    round = back ? (ref ? 3.5 + 0.0066 * x : 2.9 + 0.0028 * x) + 0.045 * p.ogroups
+                 : (ref ? 3.9 + 0.0027 * x : 2.7 + 0.00113 * x);
   return p.rounds * round;
 }
 double streamed_us(int arith, bool back, double points, bool own_velocity) {
@@ -171,18 +198,25 @@ void launch_resident(int arith, bool back, const ResidentPlan &p, ResidentArgs a
   const int nzs = std::max(a.nz - 6 - a.bx0, 1);
   a.nzs_magic = (unsigned)((1ull << 32) / nzs + 1);
   a.chunks = p.chunks;
+  a.thin = p.thin ? 1 : 0;
   a.helpers = p.helpers;
   a.cap_src = p.cap_src;
   a.cap_rec = p.cap_rec;
   a.cap_stage = p.cap_stage;
-  SWFWI_CUDA(cudaMemsetAsync(a.halo, 0, sizeof(uint4) * resident_halo(nslots, p.cps, back ? 2 : 1, p.ogroups), st));
-  if (arith == ARITH_REF) {
-    if (back) launch_t<ARITH_REF, true>(a, p.smem, st);
-    else launch_t<ARITH_REF, false>(a, p.smem, st);
-  } else {
-    if (back) launch_t<ARITH_FAST, true>(a, p.smem, st);
-    else launch_t<ARITH_FAST, false>(a, p.smem, st);
-  }
+  SWFWI_CUDA(cudaMemsetAsync(a.halo, 0, sizeof(uint4) * resident_halo(nslots, p.cps, p.rows, p.thin, back ? 2 : 1, p.ogroups),
+                             st));
+  auto go = [&](auto wide) {
+    constexpr bool W = decltype(wide)::value;
+    if (arith == ARITH_REF) {
+      if (back) launch_t<ARITH_REF, true, W>(a, p.smem, st);
+      else launch_t<ARITH_REF, false, W>(a, p.smem, st);
+    } else {
+      if (back) launch_t<ARITH_FAST, true, W>(a, p.smem, st);
+      else launch_t<ARITH_FAST, false, W>(a, p.smem, st);
+    }
+  };
+  if (p.wide) go(std::true_type());
+  else go(std::false_type());
   note_launch();
 }
 

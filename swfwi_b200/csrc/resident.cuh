@@ -26,11 +26,24 @@
 // or last group needs no neighbour).  Partly filled depth slices, which cost
 // the streaming kernels up to a quarter of their lanes, do not occur.
 //
+// Slabs of a few rows (one supershot over all SMs) leave that march a warp or
+// two a scheduler and a chain of ten loads and L + 2 rows of u2 for L rows of
+// output: 2450 (FAST) and 4500 (REF) cycles a step for a row a chunk.  The
+// two-pass form (WIDE) has an item per u2 row and depth group, then, after a
+// barrier of the compute warps, one per output row and group, u2 going
+// through shared memory: no row is formed twice and nothing is serial, for 13
+// loads a u2 item instead of 3 to 7.  (More warps than 16, or a barrier before
+// the neighbours' rows are polled, made a step slower: 1 shot of 533 x 193
+// REF 2.5 us with 512 threads, 3.1 with 768, 3.5 with 1024.)
+//
 // Edge rows travel through L2 as 8-byte {value, step tag} pairs, written by
 // the lanes that compute them and polled by the neighbour's helpers: no
 // fence, no flag and no grid barrier.  Two buffers alternate: a CTA writes
 // step n's rows only after it has received its neighbours' rows of step n-1,
-// which they computed after receiving step n-2's.  Every CTA of the grid is
+// which they computed after receiving step n-2's.  Slabs of fewer than 6 rows
+// (one shot of a small grid on all SMs) need rows of slabs further away: the
+// buffer then has a place for every row, read by whoever is within 6 of it;
+// who reads a CTA's rows is again who it reads.  Every CTA of the grid is
 // resident (cooperative launch), every wait is bounded: on timeout the CTA
 // raises the error flag, which the others' waits look at, and leaves.
 #pragma once
@@ -74,6 +87,7 @@ struct ResidentArgs {
   float dt;
   int cap_src, cap_rec, cap_stage;   // list capacities (entries)
   unsigned nzs_magic;        // 2^32 / nzs + 1: u / nzs = high word of u * nzs_magic, nzs = depths of a side strip
+  int thin;                  // slabs of fewer than 6 rows (two-pass form only): the exchange buffer is by row, not by slab
   uint4 *halo;               // zeroed before the launch
   int *err;
 };
@@ -92,7 +106,7 @@ struct ResidentSlab {
   int give_up, drawn;                       // a wait gave up; receive batches drawn
 };
 struct ResidentLayout {
-  int v, im, cf, src, rec, stage, cs, slab, args, total;
+  int v, im, cf, src, rec, stage, cs, slab, args, u2, total;   // u2: the two-pass form's, [NF][rmax+2][zp]
   __host__ __device__ ResidentLayout(bool back, int rmax, int zp, int cap_src, int cap_rec, int cap_stage) {
     v = (back ? 4 : 2) * (rmax + 12) * zp;
     im = v + rmax * zp;
@@ -103,15 +117,18 @@ struct ResidentLayout {
     cs = stage + cap_stage;
     slab = cs + kResidentChunks + 1;
     args = (slab + (int)(sizeof(ResidentSlab) / 4) + 3) / 4 * 4;   // a copy of the launch arguments
-    total = args + (int)((sizeof(ResidentArgs) + 3) / 4);
+    u2 = (args + (int)((sizeof(ResidentArgs) + 3) / 4) + 3) / 4 * 4;
+    total = u2;
   }
 };
-inline size_t resident_smem(bool backward, int rmax, int zp, int cap_src, int cap_rec, int cap_stage) {
-  return 4 * (size_t)ResidentLayout(backward, rmax, zp, cap_src, cap_rec, cap_stage).total;
+inline size_t resident_smem(bool backward, bool wide, int rmax, int zp, int cap_src, int cap_rec, int cap_stage) {
+  return 4 * ((size_t)ResidentLayout(backward, rmax, zp, cap_src, cap_rec, cap_stage).total +
+              (wide ? (backward ? 2 : 1) * (rmax + 2) * zp : 0));
 }
-// uint4 elements of the exchange buffer
-inline size_t resident_halo(int nslots, int cps, int nfields, int ogroups) {
-  return (size_t)nslots * cps * nfields * 2 * 2 * 6 * ogroups * 2;
+// uint4 elements of the exchange buffer: [slot][slab][propagation][parity]
+// [side][6][ogroups][2], or (thin) [slot][row][propagation][parity][ogroups][2]
+inline size_t resident_halo(int nslots, int cps, int rows, bool thin, int nfields, int ogroups) {
+  return (size_t)nslots * (thin ? rows : 12 * cps) * nfields * 2 * ogroups * 2;
 }
 
 namespace resident_detail {
@@ -256,7 +273,7 @@ __device__ __noinline__ void point_step(const ResidentArgs &a, float *F, int cur
 // groups a lane, taken by whichever warp is free (the helpers at once, the
 // compute warps as they finish).
 constexpr int kRecv = 2;
-template <bool BACK>
+template <bool BACK, bool WIDE>
 __device__ __noinline__ void receive_step(const ResidentArgs &a, float *F, int cur, int n) {
   constexpr int NF = BACK ? 2 : 1;
   const ResidentLayout l(BACK, a.rmax, a.zp, a.cap_src, a.cap_rec, a.cap_stage);
@@ -285,14 +302,30 @@ __device__ __noinline__ void receive_step(const ResidentArgs &a, float *F, int c
         const int sd = v >= nper ? 1 : 0, gidx = v - sd * nper;
         const bool left = has_l && sd == 0;   // rows before the slab: the left neighbour's last rows
         const int rr = (int)(((unsigned)gidx * a.omagic) >> 20), grp = gidx - rr * a.ogroups;
-        const int nb = left ? (int)blockIdx.x - 1 : (int)blockIdx.x + 1;
-        from[e] = a.halo + ((size_t)nb * NF + f) * 4 * side + ((size_t)(n & 1) * 2 + (left ? 1 : 0)) * side +
-                  (size_t)gidx * 2;
+        if (WIDE && a.thin) {
+          const int row = (left ? b.xa - 12 : b.xa + b.R - 6) + rr;   // row 0: absolute row 6
+          if (row < 0 || row >= a.nx - 12) continue;
+          from[e] = a.halo + (((size_t)b.slot * (a.nx - 12) + row) * NF + f) * 4 * a.ogroups +
+                    ((size_t)(n & 1) * a.ogroups + grp) * 2;
+        } else {
+          const int nb = left ? (int)blockIdx.x - 1 : (int)blockIdx.x + 1;
+          from[e] = a.halo + ((size_t)nb * NF + f) * 4 * side + ((size_t)(n & 1) * 2 + (left ? 1 : 0)) * side +
+                    (size_t)gidx * 2;
+        }
         to[e] = F + (2 * f + (cur ^ 1)) * field + (left ? rr : b.R + 6 + rr) * a.zp + 4 + 4 * grp;
         todo |= 1u << e;
       }
     }
     long long t0 = 0;
+    auto late = [&](int spin) {   // bounded: about a second, or until another CTA gave up
+      if ((spin & 255) != 255) return false;
+      const long long now = clock64();
+      if (t0 == 0) t0 = now;
+      if (now - t0 <= (1LL << 31) && !*(volatile int *)a.err) return false;
+      atomicExch(a.err, 1);
+      b.give_up = 1;
+      return true;
+    };
     for (int spin = 0; todo; spin++) {
       uint4 x[kRecv], y[kRecv];
 #pragma unroll
@@ -308,24 +341,158 @@ __device__ __noinline__ void receive_step(const ResidentArgs &a, float *F, int c
                                  __uint_as_float(y[e].z)));
           todo &= ~(1u << e);
         }
-      if (todo && (spin & 255) == 255) {
-        // bounded: about a second, or until another CTA gave up
-        const long long now = clock64();
-        if (t0 == 0) t0 = now;
-        if (now - t0 > (1LL << 31) || *(volatile int *)a.err) {
-          atomicExch(a.err, 1);
-          b.give_up = 1;
-          break;
-        }
-      }
+      if (todo && late(spin)) break;
     }
     __syncwarp();
   }
 }
 
+// The compute warps' part of a step in two passes (ct of cn threads).
+template <int ARITH, bool BACK>
+__device__ __forceinline__ void march_wide(const ResidentArgs &a, const ResidentLayout &l, float *F, int slot, int xa,
+                                           int R, int cur, int n, int ct, int cn) {
+  constexpr int NF = BACK ? 2 : 1;
+  const int ZP = a.zp, nz = a.nz, field = (a.rmax + 12) * ZP, G = a.ngroups, ufield = (a.rmax + 2) * ZP;
+  float *U = F + l.u2;
+  // u2 row ur (of propagation f) belongs to shared row ur + 5
+  for (int id = ct; id < NF * (R + 2) * G; id += cn) {
+    const int rr = (int)(((unsigned)id * a.gmagic) >> 20), grp = id - rr * G;
+    const int f = BACK && rr >= R + 2 ? 1 : 0, ur = rr - f * (R + 2), zg = 4 + 4 * grp;
+    const float *A = F + (2 * f + cur) * field + ur * ZP + zg;   // five rows before
+    const float *C = A + 5 * ZP;
+    float4 xm[6], xp[6];
+#pragma unroll
+    for (int k = 1; k <= 5; k++) {
+      xm[k] = ld4(A + (5 - k) * ZP);
+      xp[k] = ld4(A + (5 + k) * ZP);
+    }
+    const float4 v1 = ld4(C - 4), v2 = ld4(C), v3 = ld4(C + 4);
+    float zn[20];
+    zn[0] = zn[1] = zn[2] = zn[17] = zn[18] = zn[19] = 0.f;
+    zn[3] = C[grp > 0 ? -5 : -4];   // the first depth of the first group is no output's neighbour
+    zn[16] = C[8];
+    zn[4] = v1.x; zn[5] = v1.y; zn[6] = v1.z; zn[7] = v1.w;
+    zn[8] = v2.x; zn[9] = v2.y; zn[10] = v2.z; zn[11] = v2.w;
+    zn[12] = v3.x; zn[13] = v3.y; zn[14] = v3.z; zn[15] = v3.w;
+    float4 u;
+    if constexpr (ARITH == ARITH_FAST) {
+      const float2 lo = lap_pair_fast<0>(zn, xm, xp), hi = lap_pair_fast<1>(zn, xm, xp);
+      u = make_float4(lo.x, lo.y, hi.x, hi.y);
+    } else {
+      float uu[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        float m[6], q[6];
+        m[0] = q[0] = 0.f;
+#pragma unroll
+        for (int k = 1; k <= 5; k++) {
+          m[k] = get(xm[k], i);
+          q[k] = get(xp[k], i);
+        }
+        uu[i] = lap_pt<ARITH>(zn, i, m, q);
+      }
+      u = make_float4(uu[0], uu[1], uu[2], uu[3]);
+    }
+    st4(U + f * ufield + ur * ZP + zg, u);
+  }
+  asm volatile("bar.sync 1, %0;" ::"r"(cn) : "memory");
+
+  const bool has_l = xa > 6, has_r = xa + R < a.nx - 6;
+  const float scale = BACK ? image_scale(a.dt, a.nt - 1 - n) : 0.0f;
+  const uint32_t tag = (uint32_t)(n + 1);
+  const unsigned span = (unsigned)max(a.nx - 2 * a.ramp, 0);
+  const int O = a.ogroups;
+  for (int id = ct; id < NF * R * O; id += cn) {
+    const int rr = (int)(((unsigned)id * a.omagic) >> 20), grp = id - rr * O;
+    const int f = BACK && rr >= R ? 1 : 0, j = rr - f * R, zg = 4 + 4 * grp;
+    const bool damped = !BACK || f == 1;
+    const int at = (j + 6) * ZP + zg;
+    const float *u = U + f * ufield + (j + 1) * ZP + zg;
+    const float4 um = ld4(u - ZP), uc = ld4(u), up = ld4(u + ZP);
+    const float ucl = u[-1], ucr = u[4];
+    float *B = F + (2 * f + (cur ^ 1)) * field + at;
+    const float4 c4 = ld4(F + (2 * f + cur) * field + at), p4 = ld4(B), r4 = ld4(F + l.v + at - 6 * ZP);
+    const bool ramp_row = damped && (unsigned)(j + xa - a.ramp) >= span;
+    float4 o;
+    if constexpr (ARITH == ARITH_FAST) {
+      float2 cf0 = make_float2(2.f, 2.f), cf1 = cf0, pc0 = make_float2(-1.f, -1.f), pc1 = pc0;
+      if (damped) {
+        const float4 c = ld4(F + l.cf + zg), p = ld4(F + l.cf + ZP + zg);
+        cf0 = lo2(c);
+        cf1 = hi2(c);
+        pc0 = lo2(p);
+        pc1 = hi2(p);
+      }
+      if (ramp_row) {
+        const float2 cx = a.coef_x[xa + j];
+        if (pc0.x == -1.f) { cf0.x = cx.x; pc0.x = cx.y; }
+        if (pc0.y == -1.f) { cf0.y = cx.x; pc0.y = cx.y; }
+        if (pc1.x == -1.f) { cf1.x = cx.x; pc1.x = cx.y; }
+        if (pc1.y == -1.f) { cf1.y = cx.x; pc1.y = cx.y; }
+      }
+      const float2 o0 = update_pair_coef(lo2(c4), lo2(p4), lo2(r4), lo2(uc),
+                                         make_float2(__fadd_rn(ucl, uc.y), __fadd_rn(uc.x, uc.z)), lo2(um), lo2(up),
+                                         cf0, pc0);
+      const float2 o1 = update_pair_coef(hi2(c4), hi2(p4), hi2(r4), hi2(uc),
+                                         make_float2(__fadd_rn(uc.y, uc.w), __fadd_rn(uc.z, ucr)), hi2(um), hi2(up),
+                                         cf1, pc1);
+      o = make_float4(o0.x, o0.y, o1.x, o1.y);
+    } else {
+      const float dxr = ramp_row ? a.damp_x[xa + j] : 0.f;
+      float4 dz = make_float4(-1.f, -1.f, -1.f, -1.f);
+      if (damped) dz = ld4(F + l.cf + zg);
+      float oo[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        float delta = 0.f;
+        const float dist = get(dz, i) >= 0.f ? get(dz, i) : dxr;
+        if (damped) delta = __fmul_rn(__fmul_rn(0.05f, dist), dist);
+        oo[i] = update_pt<ARITH>(get(c4, i), get(p4, i), get(r4, i), get(uc, i), i == 0 ? ucl : get(uc, i - 1),
+                                 i == 3 ? ucr : get(uc, i + 1), get(um, i), get(up, i), delta);
+      }
+      o = make_float4(oo[0], oo[1], oo[2], oo[3]);
+    }
+    // border depths stay zero
+    o.x = zg >= 6 && zg < nz - 6 ? o.x : 0.f;
+    o.y = zg + 1 >= 6 && zg + 1 < nz - 6 ? o.y : 0.f;
+    o.z = zg + 2 < nz - 6 ? o.z : 0.f;
+    o.w = zg + 3 < nz - 6 ? o.w : 0.f;
+    st4(B, o);
+    if constexpr (BACK) {
+      if (f == 0) {
+        const float4 g4 = ld4(F + (2 + cur) * field + at);
+        float *im = F + l.im + at - 6 * ZP;
+        float4 m = ld4(im);
+        m.x = __fsub_rn(m.x, __fmul_rn(__fmul_rn(o.x, g4.x), scale));
+        m.y = __fsub_rn(m.y, __fmul_rn(__fmul_rn(o.y, g4.y), scale));
+        m.z = __fsub_rn(m.z, __fmul_rn(__fmul_rn(o.z, g4.z), scale));
+        m.w = __fsub_rn(m.w, __fmul_rn(__fmul_rn(o.w, g4.w), scale));
+        st4(im, m);
+      }
+    }
+    if (a.thin) {
+      uint4 *d = a.halo + ((((unsigned)(slot * (a.nx - 12) + xa - 6 + j) * NF + f) * 2 + (n & 1)) * O + grp) * 2;
+      put_pair2(d, o.x, o.y, tag);
+      put_pair2(d + 1, o.z, o.w, tag);
+    } else {
+      uint4 *h = a.halo + (((blockIdx.x * NF + f) * 4 + (n & 1) * 2) * (unsigned)(6 * O) + grp) * 2;
+      if (j < 6 && has_l) {
+        uint4 *d = h + (unsigned)(j * O * 2);
+        put_pair2(d, o.x, o.y, tag);
+        put_pair2(d + 1, o.z, o.w, tag);
+      }
+      if (j >= R - 6 && has_r) {
+        uint4 *d = h + (unsigned)((j - R + 12) * O * 2);
+        put_pair2(d, o.x, o.y, tag);
+        put_pair2(d + 1, o.z, o.w, tag);
+      }
+    }
+  }
+}
+
 }  // namespace resident_detail
 
-template <int ARITH, bool BACK>
+template <int ARITH, bool BACK, bool WIDE>
 __global__ void __launch_bounds__(kResidentThreads, 1) fd_resident(const __grid_constant__ ResidentArgs a) {
   using namespace resident_detail;
   constexpr int NF = BACK ? 2 : 1;   // propagations
@@ -468,7 +635,9 @@ __global__ void __launch_bounds__(kResidentThreads, 1) fd_resident(const __grid_
       __syncthreads();
     }
 
-    if (warp < cwarps) {
+    if (WIDE && warp < cwarps) {
+      march_wide<ARITH, BACK>(sa, l, F, sb.slot, xa, R, cur, n, tid, 32 * cwarps);
+    } else if (!WIDE && warp < cwarps) {
       const float scale = BACK ? image_scale(a.dt, a.nt - 1 - n) : 0.0f;
       const uint32_t tag = (uint32_t)(n + 1);
       for (int task = warp; task < NF * wtasks; task += cwarps) {
@@ -488,8 +657,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) fd_resident(const __grid_
         const float *rv = F + l.v + c0 * ZP + zg;
         const float *gc = F + (2 + cur) * field + (c0 + 6) * ZP + zg;   // receiver field at the outputs (BACK)
         float *im = F + l.im + c0 * ZP + zg;
-        // this step's place for the first edge row's group in the exchange
-        // buffer: [slot][slab][propagation][parity][side][6][ogroups][2]
+        // this step's place for the first edge row's group in the exchange buffer
         const unsigned hl = ((blockIdx.x * NF + f) * 4 + (n & 1) * 2) * (unsigned)(12 * a.ogroups) + 2 * grp;
 
         // sponge, as in the streaming kernels: the bottom ramp per depth,
@@ -662,7 +830,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) fd_resident(const __grid_
       const int hn = 32 * a.helpers;
       helper_step<BACK>(sa, F, cur, n, tid - (nthreads - hn), hn);
     }
-    if (n + 1 < a.steps && (has_l || has_r)) receive_step<BACK>(sa, F, cur, n);
+    if (n + 1 < a.steps && (has_l || has_r)) receive_step<BACK, WIDE>(sa, F, cur, n);
     if constexpr (BACK) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     cur ^= 1;

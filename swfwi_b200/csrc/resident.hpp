@@ -12,6 +12,9 @@ struct ResidentArgs;
 // `cps` CTAs a slot.
 struct ResidentPlan {
   bool ok = false;
+  bool thin = false;   // slabs of fewer than 6 rows
+  int rows = 0;        // rows a slot is cut into
+  bool wide = false;   // the two-pass form
   int rounds = 0, slots = 0, cps = 0, rmax = 0, zp = 0, ngroups = 0, ogroups = 0, chunks = 0, helpers = 0;
   int cap_src = 0, cap_rec = 0, cap_stage = 0;
   size_t smem = 0, halo = 0;   // bytes a CTA, uint4 elements of the exchange buffer
@@ -19,7 +22,7 @@ struct ResidentPlan {
 
 // src_hist / rec_hist: per padded row, the most source / receiver points any
 // slot has there.
-ResidentPlan plan_resident(bool back, int n, int nx, int nz, int bx0, bool strips, const std::vector<int> &src_hist,
+ResidentPlan plan_resident(int arith, bool back, int n, int nx, int nz, int bx0, bool strips, const std::vector<int> &src_hist,
                            const std::vector<int> &rec_hist);
 // Estimated time a step of the plan, and of the streaming kernels on a batch
 // of `points` field points (own_velocity: a velocity model per slot).
