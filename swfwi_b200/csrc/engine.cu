@@ -800,12 +800,20 @@ bool Propagator::resident_forward(Work<float> &w, int n, PointSet src, const flo
 
 bool Propagator::resident_backward(Work<float> &w, int n, PointSet src, const float *vals, long long it_stride,
                                    long long slot_stride, int i_stride, PointSet rec, int ngrec, const float *vsrc,
-                                   const float *velrcp) {
+                                   const float *velrcp, bool summed) {
   if (!resident_allowed()) return false;
   if (recon != SWFWI_RECON_STRIPS || strip_format != SWFWI_STRIP_F32) return false;
   const ResidentPlan p = plan_resident(arith, true, n, nxpad, nzpad, bx0, true, src.per_shot == 1 ? row_src1_ : row_src_,
                                        rec.pos == d_geo_pos_p_.get() ? row_geo_ : row_rec_);
   if (!resident_faster(p, true, n)) return false;
+  // Slots whose images a streamed sweep would sum step by step have an image
+  // each here, added at the end: other roundings of the same sum, as far from
+  // 64 bits.  Taken for the one or two rounds where it gains most (us a step
+  // of a gradient, resident / streamed: 2 shots of 533 x 193 7.6 / 17.2, 20
+  // shots 18.1 / 26.1; 4 shots of 993 x 343 15.9 / 21.0); at three rounds it
+  // would be 24.9 / 33.0 (24 shots of 552 x 202), but long inversions over
+  // such batches keep the sums that their recorded runs were made with.
+  if (summed && p.rounds > 2) return false;
   int steps = 0;   // the reference's loop images while t > 0.3
   for (int it = nt - 1; it >= 0 && (double)(dt * (float)it) > 0.3; it--) steps++;
   if (steps == 0) return true;
@@ -917,12 +925,9 @@ bool Propagator::run_backward(Work<T> &w, int n, PointSet src, const T *vals, lo
                               long long slot_stride, int i_stride, PointSet rec, int ngrec,
                               const T *vsrc, const void *velrcp, const std::vector<PtLine> *src_lines,
                               const std::vector<PtLine> *rec_lines, bool sum_images) {
-  // (a batch whose images are summed step by step streams: its slots' fields
-  // are in different CTAs of a resident sweep)
   if constexpr (sizeof(T) == 4) {
-    if ((n == 1 || !sum_images) &&
-        resident_backward(w, n, src, vals, it_stride, slot_stride, i_stride, rec, ngrec, vsrc,
-                          static_cast<const float *>(velrcp)))
+    if (resident_backward(w, n, src, vals, it_stride, slot_stride, i_stride, rec, ngrec, vsrc,
+                          static_cast<const float *>(velrcp), n > 1 && sum_images))
       return false;
   }
   size_t f = (size_t)n * fstride;

@@ -260,7 +260,7 @@ class Propagator {
                         const float *velrcp);
   bool resident_backward(Work<float> &w, int n, PointSet src, const float *vals, long long it_stride,
                          long long slot_stride, int i_stride, PointSet rec, int ngrec, const float *vsrc,
-                         const float *velrcp);
+                         const float *velrcp, bool summed);
   // Forward time loop for n slots.  Source values:
   // vals + it*it_stride + slot*slot_stride + i*i_stride.
   template <typename T>
@@ -273,7 +273,8 @@ class Propagator {
   // back-step also subtracts the source and images, the receiver step also
   // injects the next residual.  sum_images (FAST arithmetic, separate
   // launches only): every slot images into slot 0's image, one pass per
-  // step.  Returns true when the images were summed that way.
+  // step, unless the sweep is resident.  Returns true when the images were
+  // summed that way.
   bool run_backward(Work<T> &w, int n, PointSet src, const T *vals, long long it_stride,
                     long long slot_stride, int i_stride, PointSet rec, int ngrec, const T *vsrc,
                     const void *velrcp, const std::vector<PtLine> *src_lines = nullptr,
