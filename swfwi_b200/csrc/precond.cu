@@ -234,54 +234,67 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc(const bf16 *__restrict__ in,
 }
 
 // ---------------------------------------------------------------- 3x3 conv, tcgen05, row tiles
-// The same implicit GEMM with row-aligned tiles: the CTA's 128 pixels are
-// 16 groups of 8 consecutive pixels of one image row each.  For every group
-// the three input rows it needs (h-1, h, h+1) are staged once, 10 pixels
-// wide (the group and a one-pixel halo), as 16-byte rows per 8-channel half:
-// A(tap ky, kx) is then the staged rows of ky seen from a start address
-// shifted by kx rows, with the 8-row groups 160 B apart -- the three column
-// taps share one copy, and the input is copied 30/8 times instead of 9.
-// The rows of ky go in rounds (all three at once when they fit, else one
-// ky a round, double-buffered).
+// The same implicit GEMM with row-aligned tiles in a persistent kernel.  A
+// tile's 128 pixels are 16 groups of 8 consecutive pixels of one image row
+// each.  For every group the three input rows it needs (h-1, h, h+1) are
+// staged once, 10 pixels wide (the group and a one-pixel halo), as 16-byte
+// rows per 8-channel half: A(tap ky, kx) is then the staged rows of ky seen
+// from a start address shifted by kx rows, with the 8-row groups 160 B apart
+// -- the three column taps share one copy, and the input is copied 30/8 times
+// instead of 9.
+// A CTA keeps the weights of its output channels in shared memory and walks
+// over tiles: 320 threads copy (a thread one pixel and 8-channel half of every
+// 16 channels, no divisions beyond its group's place once a tile) into a ring
+// of stages, a stage being a tile's three rows or one of them (stage_rows), a
+// warp issues the MMAs, and four warps drain one accumulator while the next is
+// formed.  The copies bound it.  One tile a CTA with everything in turn took
+// 114 us for 16 -> 16 channels on 1.2 million pixels.
+// The MMAs of an output are those of that form in the same order (taps, then
+// channels): the same bits.
 namespace tg {
 constexpr int kGroupBytes = 160;                  // 10 pixels x 16 bytes
 constexpr int kPlaneRow = 16 * kGroupBytes;       // one ky row of the 16 groups
-__host__ __device__ inline int rows_per_round(int cin, int cout) {
-  const int kc = cin / 16;
-  if (kc * (2 * 3 * kPlaneRow + 9 * 32 * cout) <= 96 * 1024) return 3;
-  return 1;
+constexpr int kCopyThreads = 320, kThreads = kCopyThreads + 32 + 128;
+constexpr int kMaxStages = 6;
+constexpr size_t kMaxSmem = 226 * 1024;
+// output channels a CTA forms: all, or half where their weights would leave
+// no room for two stages
+__host__ __device__ inline int cols(int cin, int cout) {
+  return cin / 16 * 9 * 32 * cout > 150 * 1024 - cin / 16 * 2 * kPlaneRow && cout % 32 == 0 ? cout / 2 : cout;
 }
-__host__ __device__ inline int stage_bytes(int cin, int cout, int nky) {
-  const int kc = cin / 16;
-  return kc * (2 * nky * kPlaneRow + 3 * nky * 32 * cout);
+__host__ __device__ inline int weight_bytes(int cin, int cout) { return cin / 16 * 9 * 32 * cols(cin, cout); }
+__host__ __device__ inline int stage_rows(int cin) { return cin <= 48 ? 3 : 1; }
+__host__ __device__ inline int stage_bytes(int cin) { return cin / 16 * 2 * stage_rows(cin) * kPlaneRow; }
+// stages: as many as leave room for a second CTA where weights and two
+// stages are small, else for one
+__host__ __device__ inline int stages(int cin, int cout) {
+  const int w = weight_bytes(cin, cout), sb = stage_bytes(cin), half = 110 * 1024;
+  const int n = w + 2 * sb <= half ? (half - w) / sb : ((int)kMaxSmem - 1024 - w) / sb;
+  return n < kMaxStages ? n : kMaxStages;
+}
+__host__ __device__ inline size_t smem(int cin, int cout) {
+  return (size_t)weight_bytes(cin, cout) + (size_t)stages(cin, cout) * stage_bytes(cin) + 256;
 }
 }  // namespace tg
 
-// KC = cin / 16 is a template parameter: the staging's divisions by the
-// channel count are by constants.
+// KC = cin / 16 is a template parameter: loops by constants.
 template <bool F32, int KC>
-__global__ void __launch_bounds__(128) k_conv3x3_tg(const bf16 *__restrict__ in, const bf16 *__restrict__ w,
-                                                    const float *__restrict__ bias, void *out, int accum, int cout,
-                                                    int N, int H, int W) {
+__global__ void __launch_bounds__(tg::kThreads) k_conv3x3_tg(const bf16 *__restrict__ in, const bf16 *__restrict__ w,
+                                                             const float *__restrict__ bias, void *out, int accum,
+                                                             int cout, int N, int H, int W) {
   using namespace stream_detail;
   extern __shared__ __align__(1024) unsigned char sm[];
-  constexpr int cin = 16 * KC;
-  const int NKY = tg::rows_per_round(cin, cout), R = 3 / NKY, NS = R > 1 ? 2 : 1;
-  const int SB = tg::stage_bytes(cin, cout, NKY), ABYTES = KC * 2 * NKY * tg::kPlaneRow;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(sm + NS * SB);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 2);
-  int *gn = reinterpret_cast<int *>(bar + 3), *gh = gn + 16, *gw = gh + 16;   // the 16 groups (n = -1: none)
+  constexpr int cin = 16 * KC, NKY = KC <= 3 ? 3 : 1, R = 3 / NKY;
+  const int S = tg::stages(cin, cout), SB = tg::stage_bytes(cin), WB = tg::weight_bytes(cin, cout);
+  const int NC = tg::cols(cin, cout), co0 = blockIdx.y * NC;   // this CTA's output channels
+  uint64_t *full = reinterpret_cast<uint64_t *>(sm + WB + S * SB), *empty = full + tg::kMaxStages;
+  uint64_t *ready = empty + tg::kMaxStages, *taken = ready + 2;   // an accumulator is formed, is read
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(taken + 2);
+  volatile int *bad = reinterpret_cast<volatile int *>(tslot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int GW = (W + 7) / 8;
-  const long long groups = (long long)N * H * GW;
-  const uint32_t ncols = (uint32_t)tc::tmem_cols(cout);
-  if (tid < 16) {
-    const long long gi = (long long)blockIdx.x * 16 + tid;
-    const long long row = gi / GW;
-    gn[tid] = gi < groups ? (int)(row / H) : -1;
-    gh[tid] = gi < groups ? (int)(row % H) : 0;
-    gw[tid] = gi < groups ? (int)(gi % GW) * 8 : 0;
-  }
+  const unsigned GW = (unsigned)(W + 7) / 8, groups = (unsigned)N * H * GW;
+  const int tiles = (int)((groups + 15) / 16);
+  const uint32_t ncols = (uint32_t)tc::tmem_cols(2 * NC);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::saddr(tslot)),
                  "r"(ncols)
@@ -289,126 +302,184 @@ __global__ void __launch_bounds__(128) k_conv3x3_tg(const bf16 *__restrict__ in,
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+    for (int k = 0; k < tg::kMaxStages; k++) {
+      mbar_init(&full[k], tg::kCopyThreads);
+      mbar_init(&empty[k], 1);
+    }
+    for (int k = 0; k < 2; k++) {
+      mbar_init(&ready[k], 1);
+      mbar_init(&taken[k], 128);
+    }
+    *bad = 0;
     fence_mbar_init();
   }
+  const uint32_t sbase = tc::saddr(sm);
+  // weights: 9 taps x [kc] x NC rows in K-major core matrices
+  for (int u = tid; u < 9 * NC * 2 * KC; u += tg::kThreads) {
+    const int q = u % (2 * KC), v = u / (2 * KC), co = v % NC, tap = v / NC;
+    tc::cp16(sbase + (uint32_t)((tap * KC + (q >> 1)) * NC * 32 + ((co >> 3) * 2 + (q & 1)) * 128 + (co & 7) * 16),
+             w + ((long long)(co0 + co) * 9 + tap) * cin + q * 8, true);
+  }
+  tc::cp_commit();
+  tc::cp_wait<0>();
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t taddr = *tslot;
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(cout >> 3) << 17) | ((128u >> 4) << 24);
-  const uint32_t sbase = tc::saddr(sm);
 
-  // round rd: input rows ky = rd*NKY .. +NKY-1 and the taps 3*ky + kx
-  auto load_round = [&](int rd) {
-    const uint32_t sa = sbase + (uint32_t)((rd % NS) * SB), sb = sa + (uint32_t)ABYTES;
-    // A: [kc][half][kyl][group][10 px][16 B], 16 bytes per step along a pixel's channels
-    for (int u = tid; u < NKY * 16 * 10 * 2 * KC; u += 128) {
-      const int q = u % (2 * KC), v = u / (2 * KC), px = v % 10, gk = v / 10, g = gk & 15, kyl = gk >> 4;
-      const int n = gn[g], hh = gh[g] + rd * NKY + kyl - 1, xx = gw[g] + px - 1;
-      const bool ok = n >= 0 && hh >= 0 && hh < H && xx >= 0 && xx < W;
-      tc::cp16(sa + (uint32_t)((((q >> 1) * 2 + (q & 1)) * NKY + kyl) * tg::kPlaneRow + g * tg::kGroupBytes + px * 16),
-               ok ? in + (((long long)n * H + hh) * W + xx) * cin + q * 8 : in, ok);
-    }
-    // B: the round's 3*NKY taps x [kc] x cout rows in K-major core matrices
-    for (int u = tid; u < 3 * NKY * cout * 2 * KC; u += 128) {
-      const int q = u % (2 * KC), v = u / (2 * KC), co = v % cout, t = v / cout;
-      const int tap = rd * 3 * NKY + t;
-      tc::cp16(sb + (uint32_t)((t * KC + (q >> 1)) * cout * 32 + ((co >> 3) * 2 + (q & 1)) * 128 + (co & 7) * 16),
-               w + ((long long)co * 9 + tap) * cin + q * 8, true);
-    }
-    tc::cp_commit();
-  };
-
-  bool ok = true;
-  load_round(0);
-  for (int rd = 0; rd < R && ok; rd++) {
-    if (rd + 1 < R) {
-      if (rd >= 1 && !__syncthreads_and(mbar_wait(&bar[(rd + 1) & 1], (uint32_t)(((rd - 1) >> 1) & 1)))) {
-        ok = false;
-        break;
-      }
-      load_round(rd + 1);
-      tc::cp_wait<1>();
-    } else {
-      tc::cp_wait<0>();
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t sa = sbase + (uint32_t)((rd % NS) * SB), sb = sa + (uint32_t)ABYTES;
-      for (int t = 0; t < 3 * NKY; t++) {
-        const int kyl = t / 3, kx = t - 3 * kyl;
-        for (int kc = 0; kc < KC; kc++) {
-          // A rows: group g at g*160, row i of the group at (i + kx)*16; the
-          // channel halves NKY planes apart
-          const uint32_t a_addr = sa + (uint32_t)((kc * 2 * NKY + kyl) * tg::kPlaneRow + kx * 16);
-          const uint64_t ad = (uint64_t)((a_addr >> 4) & 0x3FFFu) |
-                              ((uint64_t)((uint32_t)(NKY * tg::kPlaneRow) >> 4) << 16) |
-                              ((uint64_t)((uint32_t)tg::kGroupBytes >> 4) << 32) | (1ull << 46);
-          const uint64_t bd = tc::kmajor_desc(sb + (uint32_t)((t * KC + kc) * cout * 32));
-          const uint32_t acc = (rd > 0 || t > 0 || kc > 0) ? 1u : 0u;
-          asm volatile(
-              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(taddr),
-              "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-              : "memory");
+  if (warp < tg::kCopyThreads / 32) {
+    // ---- copies: pixel px of group g, channels 8 * half .. of every 16
+    const int half = tid & 1, t = tid >> 1, g = t / 10, px = t - 10 * g;
+    const uint32_t dst0 = sbase + (uint32_t)(WB + half * NKY * tg::kPlaneRow + g * tg::kGroupBytes + px * 16);
+    auto landed = [&](int unit) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::saddr(&full[unit % S])) : "memory");
+    };
+    int unit = 0;
+    bool stop = false;
+    for (int tile = blockIdx.x; tile < tiles && !stop; tile += gridDim.x) {
+      const unsigned gi = (unsigned)tile * 16 + g, row = gi / GW;
+      const int n = (int)(row / (unsigned)H), h = (int)(row - (unsigned)n * H), x = (int)(gi - row * GW) * 8 + px - 1;
+      const bool col = gi < groups && x >= 0 && x < W;
+      const bf16 *src0 = in + (((long long)n * H + h - 1) * W + x) * cin + 8 * half;
+      for (int rd = 0; rd < R; rd++, unit++) {
+        const int st = unit % S;
+        if (*bad || (unit >= S && !mbar_wait(&empty[st], (uint32_t)((unit / S - 1) & 1)))) {
+          *bad = 1;
+          stop = true;
+          break;
+        }
+        const uint32_t dst = dst0 + (uint32_t)(st * SB);
+#pragma unroll
+        for (int k = 0; k < NKY; k++) {
+          const int ky = rd * NKY + k, y = h + ky - 1;
+          const bool ok = col && y >= 0 && y < H;
+          const bf16 *src = src0 + (long long)ky * W * cin;
+#pragma unroll
+          for (int kc = 0; kc < KC; kc++)
+            tc::cp16(dst + (uint32_t)((kc * 2 * NKY + k) * tg::kPlaneRow), ok ? src + 16 * kc : in, ok);
+        }
+        tc::cp_commit();
+        if (unit > 0) {
+          tc::cp_wait<1>();
+          landed(unit - 1);
         }
       }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       tc::saddr(&bar[rd & 1]))
-                   : "memory");
     }
-  }
-  if (ok && !__syncthreads_and(mbar_wait(&bar[(R - 1) & 1], (uint32_t)(((R - 1) >> 1) & 1)))) ok = false;
-  tc::cp_wait<0>();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (ok) {
-    const int r = warp * 32 + lane, g = r >> 3, i = r & 7;
-    const bool valid = gn[g] >= 0 && gw[g] + i < W;
-    const long long p = valid ? ((long long)gn[g] * H + gh[g]) * W + gw[g] + i : 0;
-    for (int c0 = 0; c0 < cout; c0 += 16) {
-      uint32_t v[16];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-            "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (valid) {
-        if constexpr (F32) {
-          float4 *o = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + p * cout + c0);
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            float4 x4 = make_float4(__uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1]),
-                                    __uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3]));
-            if (accum) {
-              const float4 q = o[k];
-              x4.x += q.x; x4.y += q.y; x4.z += q.z; x4.w += q.w;
-            }
-            o[k] = x4;
+    tc::cp_wait<0>();
+    if (unit > 0) landed(unit - 1);
+  } else if (warp == tg::kCopyThreads / 32) {
+    // ---- MMAs
+    if (lane == 0) {
+      // kind::f16: FP32 accumulator, BF16 A and B, both K-major, N = NC, M = 128
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NC >> 3) << 17) | ((128u >> 4) << 24);
+      int unit = 0, k = 0;
+      bool stop = false;
+      for (int tile = blockIdx.x; tile < tiles && !stop; tile += gridDim.x, k++) {
+        const int buf = k & 1;
+        if (*bad || (k >= 2 && !mbar_wait(&taken[buf], (uint32_t)((k / 2 - 1) & 1)))) {
+          *bad = 1;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc0 = taddr + (uint32_t)(buf * NC);
+        for (int rd = 0; rd < R; rd++, unit++) {
+          const int st = unit % S;
+          if (*bad || !mbar_wait(&full[st], (uint32_t)((unit / S) & 1))) {
+            *bad = 1;
+            stop = true;
+            break;
           }
-        } else {
-          uint4 *o = reinterpret_cast<uint4 *>(reinterpret_cast<bf16 *>(out) + p * cout + c0);
-          uint32_t pk[8];
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t sa = sbase + (uint32_t)(WB + st * SB);
+          for (int t = 0; t < 3 * NKY; t++) {
+            const int kyl = t / 3, kx = t - 3 * kyl;
+            for (int kc = 0; kc < KC; kc++) {
+              // A rows: group g at g*160, row i of the group at (i + kx)*16;
+              // the channel halves NKY planes apart
+              const uint32_t a_addr = sa + (uint32_t)((kc * 2 * NKY + kyl) * tg::kPlaneRow + kx * 16);
+              const uint64_t ad = (uint64_t)((a_addr >> 4) & 0x3FFFu) |
+                                  ((uint64_t)((uint32_t)(NKY * tg::kPlaneRow) >> 4) << 16) |
+                                  ((uint64_t)((uint32_t)tg::kGroupBytes >> 4) << 32) | (1ull << 46);
+              const uint64_t bd = tc::kmajor_desc(sbase + (uint32_t)(((rd * 3 * NKY + t) * KC + kc) * NC * 32));
+              const uint32_t acc = (rd > 0 || t > 0 || kc > 0) ? 1u : 0u;
+              asm volatile(
+                  "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(acc0),
+                  "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+                  : "memory");
+            }
+          }
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                           tc::saddr(&empty[st]))
+                       : "memory");
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         tc::saddr(&ready[buf]))
+                     : "memory");
+      }
+      // a wait gave up: bounded, the MMAs still in flight
+      if (*bad && k > 0) mbar_wait(&ready[(k - 1) & 1], (uint32_t)(((k - 1) / 2) & 1));
+    }
+    __syncwarp();
+  } else {
+    // ---- epilogue: warp q holds the tensor-memory lanes 32 q .., q = warp % 4
+    const int q = warp & 3, r = q * 32 + lane, g = r >> 3, i = r & 7;
+    int k = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, k++) {
+      const int buf = k & 1;
+      const unsigned gi = (unsigned)tile * 16 + g, row = gi / GW;
+      const int x = (int)(gi - row * GW) * 8 + i;
+      const bool valid = gi < groups && x < W;
+      const long long p = valid ? (long long)row * W + x : 0;
+      const bool got = mbar_wait(&ready[buf], (uint32_t)((k / 2) & 1));
+      if (!got) *bad = 1;
+      if (!__all_sync(0xffffffffu, got) || *bad) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int c0 = 0; c0 < NC; c0 += 16) {
+        uint32_t v[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(taddr + (uint32_t)(buf * NC) + ((uint32_t)(q * 32) << 16) + (uint32_t)c0));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (c0 + 16 >= NC) {   // the accumulator is read: the MMAs may have it back
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::saddr(&taken[buf])) : "memory");
+        }
+        if (valid) {
+          if constexpr (F32) {
+            float4 *o = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + p * cout + co0 + c0);
 #pragma unroll
-          for (int k = 0; k < 8; k++)
-            pk[k] = pack_bf16(fmaxf(__uint_as_float(v[2 * k]) + bias[c0 + 2 * k], 0.0f),
-                              fmaxf(__uint_as_float(v[2 * k + 1]) + bias[c0 + 2 * k + 1], 0.0f));
-          o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+            for (int e = 0; e < 4; e++) {
+              float4 x4 = make_float4(__uint_as_float(v[4 * e]), __uint_as_float(v[4 * e + 1]),
+                                      __uint_as_float(v[4 * e + 2]), __uint_as_float(v[4 * e + 3]));
+              if (accum) {
+                const float4 b = o[e];
+                x4.x += b.x; x4.y += b.y; x4.z += b.z; x4.w += b.w;
+              }
+              o[e] = x4;
+            }
+          } else {
+            uint4 *o = reinterpret_cast<uint4 *>(reinterpret_cast<bf16 *>(out) + p * cout + co0 + c0);
+            const float *bs = bias + co0 + c0;
+            uint32_t pk[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+              pk[e] = pack_bf16(fmaxf(__uint_as_float(v[2 * e]) + bs[2 * e], 0.0f),
+                                fmaxf(__uint_as_float(v[2 * e + 1]) + bs[2 * e + 1], 0.0f));
+            o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+          }
         }
       }
     }
-  } else if (tid == 0) {
-    atomicExch(&g_conv_timeout, 1);
-    mbar_wait(&bar[0], 0u);   // bounded: whatever MMAs are still in flight
-    mbar_wait(&bar[1], 1u);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (tid == 0 && *bad) atomicExch(&g_conv_timeout, 1);
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
@@ -1161,13 +1232,11 @@ dim3 row_grid(int C, int rows, int W) {
 
 }  // namespace
 
+// Dynamic shared memory, raised where needed so that no more CTAs are
+// resident on an SM than its tensor memory holds.
 size_t conv_tg_smem(int cin, int cout) {
-  const int nky = tg::rows_per_round(cin, cout);
-  const size_t need = (nky == 3 ? 1 : 2) * (size_t)tg::stage_bytes(cin, cout, nky) + 24 + 3 * 16 * 4 + 8;
-  const int fit = 512 / tc::tmem_cols(cout);
-  if (fit >= 16) return need;
-  const size_t cap = 228 * 1024 / (fit + 1) - 1024 + 16;
-  return std::max(need, cap);
+  const int fit = 512 / tc::tmem_cols(2 * tg::cols(cin, cout));   // CTAs whose accumulators fit
+  return std::max(tg::smem(cin, cout), (size_t)(228 * 1024 / (fit + 1) - 1024 + 16));
 }
 
 template <bool F32, int KC>
@@ -1179,8 +1248,13 @@ void conv_tg_kc(const bf16 *in, const bf16 *w, const float *bias, void *out, boo
     return true;
   }();
   (void)attr;
-  const long long groups = (long long)N * H * ((W + 7) / 8);
-  k_conv3x3_tg<F32, KC><<<(unsigned)((groups + 15) / 16), 128, conv_tg_smem(16 * KC, cout), st>>>(
+  const long long tiles = ((long long)N * H * ((W + 7) / 8) + 15) / 16;
+  const size_t smem = conv_tg_smem(16 * KC, cout);
+  const int halves = cout / tg::cols(16 * KC, cout);
+  const long long ctas = std::max(1LL, (smem <= 112 * 1024 ? 296LL : 148LL) / halves);   // one or two an SM
+  // tiles evenly over the CTAs
+  const long long per = (tiles + ctas - 1) / ctas;
+  k_conv3x3_tg<F32, KC><<<dim3((unsigned)((tiles + per - 1) / per), (unsigned)halves), tg::kThreads, smem, st>>>(
       in, w, bias, out, accum ? 1 : 0, cout, N, H, W);
   noted();
 }
@@ -1206,9 +1280,9 @@ void launch_conv3x3(const bf16 *in, int cin, const bf16 *w, const float *bias, v
                 "conv widths must be multiples of 16, at most 128 in and 256 out");
   SWFWI_REQUIRE(N > 0 && H > 0 && W > 0, "conv image size out of range");
   SWFWI_REQUIRE(out_f32 || bias, "BF16 conv output needs a bias");
-  // row tiles (each input row staged once) where their stages fit twice on
-  // an SM, else the pixel-run tiles
-  const bool rows = conv_tg_smem(cin, cout) <= 100 * 1024;
+  // row tiles (each input row staged once) where weights and two stages fit,
+  // and their group index 32 bits; else the pixel-run tiles
+  const bool rows = tg::stages(cin, cout) >= 2 && (long long)N * H * ((W + 7) / 8) < (1LL << 31) - 32;
   if (out_f32) {
     if (!(rows && conv_tg_go<true>(in, cin, w, bias, out, accum, cout, N, H, W, st)))
       conv_tc_go<true>(in, cin, w, bias, out, accum, cout, N, H, W, st);
