@@ -91,8 +91,9 @@ void launch_t(const ResidentArgs &a, size_t smem, cudaStream_t st) {
 
 }  // namespace
 
-static ResidentPlan plan_slabs(bool thin, int arith, bool back, int n, int nx, int nz, int bx0, bool strips, const std::vector<int> &src_hist,
-                           const std::vector<int> &rec_hist) {
+// thin: slabs may have fewer than 6 rows
+static ResidentPlan plan_slabs(bool thin, int arith, bool back, int n, int nx, int nz, int bx0, bool strips,
+                               const std::vector<int> &src_hist, const std::vector<int> &rec_hist) {
   ResidentPlan p;
   const int rows = nx - 12;
   if (n <= 0 || rows < 1 || nz < 16) return p;
@@ -203,8 +204,8 @@ void launch_resident(int arith, bool back, const ResidentPlan &p, ResidentArgs a
   a.cap_src = p.cap_src;
   a.cap_rec = p.cap_rec;
   a.cap_stage = p.cap_stage;
-  SWFWI_CUDA(cudaMemsetAsync(a.halo, 0, sizeof(uint4) * resident_halo(nslots, p.cps, p.rows, p.thin, back ? 2 : 1, p.ogroups),
-                             st));
+  const size_t halo = resident_halo(nslots, p.cps, p.rows, p.thin, back ? 2 : 1, p.ogroups);
+  SWFWI_CUDA(cudaMemsetAsync(a.halo, 0, sizeof(uint4) * halo, st));
   auto go = [&](auto wide) {
     constexpr bool W = decltype(wide)::value;
     if (arith == ARITH_REF) {

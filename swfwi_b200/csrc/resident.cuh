@@ -87,7 +87,7 @@ struct ResidentArgs {
   float dt;
   int cap_src, cap_rec, cap_stage;   // list capacities (entries)
   unsigned nzs_magic;        // 2^32 / nzs + 1: u / nzs = high word of u * nzs_magic, nzs = depths of a side strip
-  int thin;                  // slabs of fewer than 6 rows (two-pass form only): the exchange buffer is by row, not by slab
+  int thin;                  // slabs of fewer than 6 rows (two-pass form only): exchange buffer by row, not by slab
   uint4 *halo;               // zeroed before the launch
   int *err;
 };
