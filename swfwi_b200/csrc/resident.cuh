@@ -36,9 +36,9 @@
 // the neighbours' rows are polled, made a step slower: 1 shot of 533 x 193
 // REF 2.5 us with 512 threads, 3.1 with 768, 3.5 with 1024.)
 //
-// Edge rows travel through L2 as 8-byte {value, step tag} pairs, written by
-// the lanes that compute them and polled by the neighbour's helpers: no
-// fence, no flag and no grid barrier.  Two buffers alternate: a CTA writes
+// Edge rows travel through L2 as 8-byte {value, step tag} pairs, each one
+// 64-bit access, written by the lanes that compute them and polled by the
+// neighbour's helpers: no fence, no flag and no grid barrier.  Two buffers alternate: a CTA writes
 // step n's rows only after it has received its neighbours' rows of step n-1,
 // which they computed after receiving step n-2's.  Slabs of fewer than 6 rows
 // (one shot of a small grid on all SMs) need rows of slabs further away: the
@@ -134,18 +134,20 @@ inline size_t resident_halo(int nslots, int cps, int rows, bool thin, int nfield
 namespace resident_detail {
 using namespace stream_detail;
 
+// Two pairs a 16-byte access.  Each pair is one 64-bit element of it: the
+// memory model makes an element of a vector access one scalar access, so a
+// value and its tag cannot be seen apart (as four 32-bit elements they could).
+__device__ __forceinline__ unsigned long long pair_of(float v, uint32_t tag) {
+  return (unsigned long long)tag << 32 | __float_as_uint(v);
+}
 __device__ __forceinline__ void put_pair2(uint4 *dst, float a, float b, uint32_t tag) {
-  asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "r"(__float_as_uint(a)), "r"(tag),
-               "r"(__float_as_uint(b)), "r"(tag)
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(dst), "l"(pair_of(a, tag)), "l"(pair_of(b, tag))
                : "memory");
 }
 __device__ __forceinline__ uint4 get_pair2(const uint4 *src) {
-  uint4 v;
-  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(src)
-               : "memory");
-  return v;
+  unsigned long long a, b;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(src) : "memory");
+  return make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
 }
 __device__ __forceinline__ void cp4(uint32_t dst, const float *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
