@@ -162,7 +162,7 @@ __device__ __forceinline__ float image_scale(float dt, int it) {
   return (double)t > 0.4 ? 1.0f : (float)(((double)t - 0.3) / 0.1);
 }
 
-// Boundary strip cell e of a slab (backward: its halo rows too): 6 below the
+// Boundary strip cell e of a slab (its rows in reach): 6 below the
 // model for the rows [bx0-6, nx-bx0+6), then the depths [6, nz-bx0) of the 6
 // rows left and of the 6 rows right of the model.  g: its index in a step's
 // strip, o: its shared offset.  Each of the three runs is contiguous in g.
@@ -514,7 +514,11 @@ __global__ void __launch_bounds__(kResidentThreads, 1) fd_resident(const __grid_
     const int s0 = slab_first(a.nx - 12, a.cps, slab), R = slab_first(a.nx - 12, a.cps, slab + 1) - s0, xa = 6 + s0;
     if (tid == 0) {
       sa = a;
-      const int w = 6, b0 = a.bx0, ra = BACK ? xa - 6 : xa, rb = BACK ? xa + R + 6 : xa + R;
+      // strip rows in reach: going back the halo rows too, forward the own
+      // rows and, of a sponge of fewer than 6 points, the rows outside the
+      // computing zone (their cells stay zero)
+      const int w = 6, b0 = a.bx0, ra = BACK || slab == 0 ? xa - 6 : xa,
+                rb = BACK || slab == a.cps - 1 ? xa + R + 6 : xa + R;
       sb.slot = slot;
       sb.R = R;
       sb.xa = xa;
