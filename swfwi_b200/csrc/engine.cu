@@ -372,6 +372,11 @@ void Propagator::upload_geometry() {
     row_src_[sx[i]]++;
   }
   for (int i = 0; i < ng; i++) row_geo_[gxp[i]]++;
+  src_in_strips_ = false;
+  for (int i = 0; i < ns; i++)
+    if (sx[i] >= bx0 - 6 && sx[i] < nxpad - bx0 + 6 && sz[i] < nzpad - bx0 + 6 &&
+        (sz[i] >= nzpad - bx0 || sx[i] < bx0 || sx[i] >= nxpad - bx0))
+      src_in_strips_ = true;
   rec_unused_ = false;
   for (int s = 0; s < ns; s++) {
     std::vector<int> h(nxpad, 0);
@@ -1067,8 +1072,9 @@ bool Propagator::run_backward(Work<T> &w, int n, PointSet src, const T *vals, lo
   loop_key_common(key);
   // With the summed image (interior cells only), step it-1's FP32 strip
   // restore, which writes boundary cells of the field the source
-  // subtraction of step it writes, rides in that launch.
-  const bool fold_strips = summed && strip_format == SWFWI_STRIP_F32;
+  // subtraction of step it writes, rides in that launch; a source that lies
+  // in the strips has to be subtracted first and overwritten then.
+  const bool fold_strips = summed && strip_format == SWFWI_STRIP_F32 && !src_in_strips_;
   run_loop(1, (double)n * nxpad * nzpad, key, [&] {
   if (fold_strips)
     launch_strip_read<T>(w.strips.get() + (long long)(nt - 1) * bsize, bstride, sp0, fstride, n, nxpad, nzpad, bx0,

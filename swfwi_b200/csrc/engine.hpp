@@ -211,6 +211,7 @@ class Propagator {
   // sources, one shot's receivers, the common receiver line
   std::vector<int> row_src1_, row_src_, row_rec_, row_geo_;
   bool rec_unused_ = false;     // some shots have fewer than ngmax receivers
+  bool src_in_strips_ = false;  // some source is a cell of the boundary strips
   DevBuf<uint4> res_halo_;      // edge rows of the resident time loop
   cudaStream_t st_ = nullptr;   // 0 = the legacy default stream
   const float *vel_ = nullptr;

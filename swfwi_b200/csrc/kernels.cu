@@ -239,6 +239,7 @@ __global__ void k_inject2(T *fa, PointSet pa, const T *va, long long va_slot_str
   const int bshot = pb.slot_shot ? pb.slot_shot[slot] : slot;
   // as k_after_forward: all loads of a thread's elements before its stores;
   // the strip band and the source and receiver points are disjoint cells
+  // (the caller gives no strips where a source lies in them)
   for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < most; i0 += kSmallE * stride) {
     int ap[kSmallE], bp[kSmallE];
 #pragma unroll
