@@ -103,6 +103,7 @@ struct ResidentSlab {
   int slot, R, xa;                          // own rows xa .. xa+R-1; shared row r is absolute row xa-6+r
   int nsrc, nrec;
   int nstrip, nbot, bot0, nlft, lft0, rgt0;   // strip cells in reach, see strip_cell
+  int band;                                 // backward: a source in reach is a strip cell
   int give_up, drawn;                       // a wait gave up; receive batches drawn
 };
 struct ResidentLayout {
@@ -231,9 +232,17 @@ __device__ __noinline__ void helper_step(const ResidentArgs &a, float *F, int cu
   }
 }
 
+// True where a strip has a cell: the 6 rows and depths around the model.
+__device__ __forceinline__ bool in_strips(const ResidentArgs &a, int x, int z) {
+  const int b0 = a.bx0;
+  if (x < b0 - 6 || x >= a.nx - b0 + 6 || z < 6 || z >= a.nz - b0 + 6) return false;
+  return z >= a.nz - b0 || x < b0 || x >= a.nx - b0;
+}
+
 // The points of the current fields before a step's march: sources in
 // (forward); the last step's sources out of the rebuilt field, its image at
-// them, the strips and the receiver sources in (backward).
+// them, the strips and the receiver sources in (backward).  A source that
+// lies in the strips is imaged, then overwritten by them.
 template <bool BACK>
 __device__ __noinline__ void point_step(const ResidentArgs &a, float *F, int cur, int n) {
   const ResidentLayout l(BACK, a.rmax, a.zp, a.cap_src, a.cap_rec, a.cap_stage);
@@ -257,6 +266,7 @@ __device__ __noinline__ void point_step(const ResidentArgs &a, float *F, int cur
         src_img[k] = __fsub_rn(src_img[k], __fmul_rn(__fmul_rn(v, F[(2 + (cur ^ 1)) * field + src_off[k]]), scale));
       }
     }
+    if (b.band) __syncthreads();
     for (int e = tid; e < b.nstrip; e += nthreads) {
       int g, o;
       strip_cell(a, b, e, g, o);
@@ -530,6 +540,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) fd_resident(const __grid_
       sb.rgt0 = max(ra, a.nx - b0);
       const int nrgt = max(min(rb, a.nx - b0 + w) - sb.rgt0, 0);
       sb.nstrip = a.strips ? sb.nbot * w + (sb.nlft + nrgt) * max(nz - 6 - b0, 0) : 0;
+      sb.band = 0;
       sb.give_up = 0;
       sb.drawn = 0;
     }
@@ -576,6 +587,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) fd_resident(const __grid_
       if (p < 0) continue;
       const int x = p / a.pitch, z = p - x * a.pitch, r = x - (xa - 6);
       if (r < 0 || r >= R + 12) continue;
+      if (BACK && in_strips(a, x, z)) sb.band = 1;
       const int k = atomicAdd(&sb.nsrc, 1);
       if (k < a.cap_src) {
         src_off[k] = r * ZP + z;

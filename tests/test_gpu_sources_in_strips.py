@@ -10,6 +10,7 @@ import pytest
 
 from swfwi_b200.survey import Survey, layered_model
 from tests.conftest import rel_l2
+from tests.test_gpu_resident import sweep
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +44,14 @@ def test_streamed_batch_gradient(cuda, where, shots):
         out.append(grad.cpu().numpy())
     # the FAST arithmetic's bound on gradients
     assert rel_l2(out[0], out[1]) < 1e-4
+
+
+@pytest.mark.parametrize("arith", [0, 1])
+@pytest.mark.parametrize("where", PLACES)
+@pytest.mark.parametrize("nb", [8, 10])
+def test_resident_sweeps(cuda, arith, where, nb):
+    """The resident sweep, which does both in one phase of a step, against
+    the streaming kernels: the same bits."""
+    s = survey(where, nb)
+    for a, b in zip(sweep(cuda, s, arith, False), sweep(cuda, s, arith, True)):
+        assert cuda.equal(a, b)
