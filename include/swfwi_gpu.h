@@ -361,6 +361,9 @@ int swfwi_prtm2d_set_adjoint(swfwi_prtm *h, int mode);
  * and adjoint mode replays its time loops as one CUDA graph (captured on
  * the second such call); 0: every call launches its kernels one by one. */
 int swfwi_prtm2d_set_graphs(swfwi_prtm *h, int on);
+/* on = 1 (default): sweeps run as one launch with their fields on chip where
+ * the grid allows it; 0: as the launched time loops (set_graphs). */
+int swfwi_prtm2d_set_resident(swfwi_prtm *h, int on);
 /* shots one launch sequence carries (1 for REF) */
 int swfwi_prtm2d_batch(swfwi_prtm *h, int *shots);
 /* prtm2d_lop (:354-437): adj = 0: dat += L mod (Born); adj = 1: mod += L'

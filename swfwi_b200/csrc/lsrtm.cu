@@ -481,6 +481,7 @@ class Prtm {
     adj_mode_ = m;
   }
   void set_graphs(bool on) { use_graphs_ = on; }
+  void set_resident(bool on) { use_resident_ = on; }
 
   // prtm2d_lop (:354-437) on device arrays.  A call that repeats an earlier
   // one's arrays, direction and mode replays the time loops as one CUDA
@@ -608,6 +609,7 @@ class Prtm {
     return p;
   }
   bool resident(bool adj) const {
+    if (!use_resident_) return false;
     if (!adj) return plan_[PRTM_BORN].ok;
     return plan_[PRTM_SOURCE].ok && plan_[adj_mode_ == SWFWI_PRTM_ADJ_EXACT ? PRTM_TRANSPOSE : PRTM_MIGRATE].ok;
   }
@@ -890,7 +892,7 @@ class Prtm {
 
   int arith_, nz_, nx_, nb_, nt_, ns_, ng_, nzpad_ = 0, nxpad_ = 0;
   int kmax_ = 1, adj_mode_ = SWFWI_PRTM_ADJ_REFERENCE;
-  bool g_swapped_ = false, use_graphs_ = true, geo_serial_ = false;
+  bool g_swapped_ = false, use_graphs_ = true, use_resident_ = true, geo_serial_ = false;
   int sms_ = 148;
   PrtmPlan plan_[4];               // by PrtmSweep
   std::vector<int> row_rec_;
@@ -938,6 +940,13 @@ extern "C" int swfwi_prtm2d_set_graphs(swfwi_prtm *h, int on) {
   return guarded([&] {
     SWFWI_REQUIRE(h && h->p, "null handle");
     h->p->set_graphs(on != 0);
+  });
+}
+
+extern "C" int swfwi_prtm2d_set_resident(swfwi_prtm *h, int on) {
+  return guarded([&] {
+    SWFWI_REQUIRE(h && h->p, "null handle");
+    h->p->set_resident(on != 0);
   });
 }
 

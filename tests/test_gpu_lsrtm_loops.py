@@ -1,0 +1,87 @@
+"""The LSRTM operator's two forms, on-chip sweeps and launched time loops: the
+form that set_resident asks for is the one that runs, the launched loops replay
+as graphs with the same bits and counts, and the forms agree: bit for bit in
+the reference arithmetic, also where calls alternate between them (the Born
+branch continues from the fields of the call before)."""
+import numpy as np
+import pytest
+
+from tests.conftest import rel_l2
+from tests.gpu_helpers import t
+from tests.test_gpu_lsrtm import _op
+
+pytestmark = pytest.mark.gpu
+
+
+def calls(torch, op, g, modes, launched=None):
+    """Two rounds of modelling and migration; launched(i): whether call i
+    takes the launched loops."""
+    mod, dat = t(torch, g["line_mod"]), t(torch, g["line_dat"])
+    b, m = torch.zeros_like(dat), torch.zeros_like(mod)
+    out = []
+    for mode in modes:
+        op.set_adjoint(mode)
+        for _ in range(3):
+            for adj in (False, True):
+                if launched is not None:
+                    op.set_resident(not launched(len(out)))
+                op.lop(adj, False, m if adj else mod, dat if adj else b)
+                out.append((m if adj else b).cpu().numpy().copy())
+    return out
+
+
+@pytest.mark.parametrize("arith", [0, 1])
+def test_launched_loops_replay_bit_identical(cuda, arith):
+    import swfwi_b200 as S
+    outs, counts = [], []
+    for graphs in (True, False):
+        op, g = _op(cuda, "line", arith)
+        op.set_resident(False)
+        op.set_graphs(graphs)
+        cuda.cuda.synchronize()
+        S.stats_reset()
+        outs.append(calls(cuda, op, g, (S.PRTM_ADJ_REFERENCE, S.PRTM_ADJ_EXACT)))
+        counts.append(S.stats_read()["kernel_launches"])
+        op.close()
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
+    assert counts[0] == counts[1]
+    assert counts[0] > 12 * 2 * g["line_dat"].shape[-1]     # launches every step
+
+
+@pytest.mark.parametrize("arith", [0, 1])
+def test_on_chip_sweeps_are_few_launches(cuda, arith):
+    import swfwi_b200 as S
+    op, g = _op(cuda, "line", arith)
+    cuda.cuda.synchronize()
+    S.stats_reset()
+    calls(cuda, op, g, (S.PRTM_ADJ_REFERENCE, S.PRTM_ADJ_EXACT))
+    shots = g["line_dat"].shape[0] if arith == S.ARITH_REF else 1
+    assert S.stats_read()["kernel_launches"] <= 12 * 3 * shots
+    op.close()
+
+
+@pytest.mark.parametrize("pattern", ["never", "always", "every other", "first half"])
+def test_forms_agree_bit_for_bit_in_reference_arithmetic(cuda, pattern):
+    import swfwi_b200 as S
+    pick = {"never": lambda i: False, "always": lambda i: True, "every other": lambda i: i % 2 == 0,
+            "first half": lambda i: i < 6}[pattern]
+    outs = []
+    for launched in (lambda i: True, pick):
+        op, g = _op(cuda, "line", S.ARITH_REF)
+        outs.append(calls(cuda, op, g, (S.PRTM_ADJ_REFERENCE, S.PRTM_ADJ_EXACT), launched))
+        op.close()
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_forms_agree_in_fast_arithmetic(cuda):
+    import swfwi_b200 as S
+    outs = []
+    for on in (True, False):
+        op, g = _op(cuda, "line", S.ARITH_FAST)
+        op.set_resident(on)
+        outs.append(calls(cuda, op, g, (S.PRTM_ADJ_REFERENCE, S.PRTM_ADJ_EXACT)))
+        op.close()
+    for a, b in zip(*outs):     # each within the FAST bound of 64 bits
+        assert rel_l2(a, b) < 2e-4
