@@ -241,7 +241,10 @@ __global__ void __launch_bounds__(kPrtmThreads, 1) k_prtm_resident(const __grid_
     const int xa = 2 + s0;
     if (tid == 0) {
       sa = a;
-      const int ra = BACKW ? xa - 2 : xa, rb = BACKW ? xa + R + 2 : xa + R;   // ring rows in reach
+      // ring rows in reach: going back the halo rows too, forward the own
+      // rows and, of a sponge of fewer than 4 cells, the grid's outer rows
+      // (their cells stay zero)
+      const int ra = BACKW || slab == 0 ? xa - 2 : xa, rb = BACKW || slab == a.cps - 1 ? xa + R + 2 : xa + R;
       sb.slot = slot;
       sb.R = R;
       sb.xa = xa;

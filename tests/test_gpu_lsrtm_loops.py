@@ -3,6 +3,8 @@ form that set_resident asks for is the one that runs, the launched loops replay
 as graphs with the same bits and counts, and the forms agree: bit for bit in
 the reference arithmetic, also where calls alternate between them (the Born
 branch continues from the fields of the call before)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -85,3 +87,49 @@ def test_forms_agree_in_fast_arithmetic(cuda):
         op.close()
     for a, b in zip(*outs):     # each within the FAST bound of 64 bits
         assert rel_l2(a, b) < 2e-4
+
+
+def stale_blocks(torch, size, n=64):
+    """Frees every other of n device blocks of `size` bytes filled with 12.08f,
+    so that allocations of that size find them; returns the others, to be
+    freed by the caller (the driver clears memory that it maps anew)."""
+    rt = ctypes.CDLL("libcudart.so.12")
+    blocks = []
+    for _ in range(n):
+        p = ctypes.c_void_p()
+        assert rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(size)) == 0
+        assert rt.cudaMemset(p, 0x41, ctypes.c_size_t(size)) == 0
+        blocks.append(p)
+    torch.cuda.synchronize()
+    for p in blocks[::2]:
+        assert rt.cudaFree(p) == 0
+    return rt, blocks[1::2]
+
+
+@pytest.mark.parametrize("arith", [0, 1])
+@pytest.mark.parametrize("nb", [2, 3, 4])
+def test_thin_sponge_ring_is_saved_whole(cuda, arith, nb):
+    """With a sponge of 2 or 3 cells the saved ring has cells in the grid's
+    outer rows: they have to be written too, or the migration restores what
+    the memory held before."""
+    import swfwi_b200 as S
+    nx, nz, nt, ng = 24, 16, 200, 12
+    rng = np.random.default_rng(nb)
+    vel = t(cuda, rng.uniform(1500, 2500, (nx, nz)).astype(np.float32))
+    dat = t(cuda, rng.standard_normal((1, ng, nt)).astype(np.float32))
+    out = []
+    for resident in (False, True):
+        rt, kept = stale_blocks(cuda, nt * 4 * (nx + nz) * 4)
+        op = S.Prtm2d(vel, dz=10.0, dx=10.0, dt=0.001, amp=1.0, fm=25.0, nb=nb, nt=nt, ns=1, ng=ng, sxbeg=12, szbeg=8,
+                      jsx=0, jsz=0, gxbeg=0, gzbeg=2, jgx=2, jgz=0, arith=arith)
+        op.set_resident(resident)
+        m = cuda.zeros((nx, nz), device="cuda")
+        op.lop(True, False, m, dat)
+        out.append(m.cpu().numpy())
+        op.close()
+        for p in kept:
+            rt.cudaFree(p)
+    if arith == S.ARITH_REF:
+        np.testing.assert_array_equal(out[1], out[0])
+    else:
+        assert rel_l2(out[1], out[0]) < 2e-4
