@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstring>
 #include <random>
+#include "conv_tiles.hpp"
 #include "kernels.cuh"
 #include "precond.hpp"
 #include "stream.cuh"
@@ -85,7 +86,6 @@ __device__ __forceinline__ uint64_t kmajor_desc(uint32_t addr) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(256u >> 4) << 32) |
          (1ull << 46);
 }
-__host__ __device__ inline int tmem_cols(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : 256)); }
 // 16 bytes global -> shared, zero-filled when !valid (src is then not read)
 __device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc(const bf16 *__restrict__ in,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long HW = (long long)H * W, P = (long long)N * HW;
   const long long p0 = (long long)blockIdx.x * 128;
-  const uint32_t ncols = (uint32_t)tc::tmem_cols(cout);
+  const uint32_t ncols = (uint32_t)tmem_cols(cout);
   // thread tid copies A row tid (its pixel, decoded once; valid = inside the
   // batch) and the B rows co = tid, tid + 128, ... of every tap
   const long long pm = p0 + tid;
@@ -274,31 +274,6 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc(const bf16 *__restrict__ in,
 // 114 us for 16 -> 16 channels on 1.2 million pixels.
 // The MMAs of an output are those of that form in the same order (taps, then
 // channels): the same bits.
-namespace tg {
-constexpr int kGroupBytes = 160;                  // 10 pixels x 16 bytes
-constexpr int kPlaneRow = 16 * kGroupBytes;       // one ky row of the 16 groups
-constexpr int kCopyThreads = 320, kThreads = kCopyThreads + 32 + 128;
-constexpr int kMaxStages = 6;
-constexpr size_t kMaxSmem = 226 * 1024;
-// output channels a CTA forms: all, or half where their weights would leave
-// no room for two stages
-__host__ __device__ inline int cols(int cin, int cout) {
-  return cin / 16 * 9 * 32 * cout > 150 * 1024 - cin / 16 * 2 * kPlaneRow && cout % 32 == 0 ? cout / 2 : cout;
-}
-__host__ __device__ inline int weight_bytes(int cin, int cout) { return cin / 16 * 9 * 32 * cols(cin, cout); }
-__host__ __device__ inline int stage_rows(int cin) { return cin <= 48 ? 3 : 1; }
-__host__ __device__ inline int stage_bytes(int cin) { return cin / 16 * 2 * stage_rows(cin) * kPlaneRow; }
-// stages: as many as leave room for a second CTA where weights and two
-// stages are small, else for one
-__host__ __device__ inline int stages(int cin, int cout) {
-  const int w = weight_bytes(cin, cout), sb = stage_bytes(cin), half = 110 * 1024;
-  const int n = w + 2 * sb <= half ? (half - w) / sb : ((int)kMaxSmem - 1024 - w) / sb;
-  return n < kMaxStages ? n : kMaxStages;
-}
-__host__ __device__ inline size_t smem(int cin, int cout) {
-  return (size_t)weight_bytes(cin, cout) + (size_t)stages(cin, cout) * stage_bytes(cin) + 256;
-}
-}  // namespace tg
 
 // KC = cin / 16 is a template parameter: loops by constants.
 template <bool F32, int KC>
@@ -317,7 +292,7 @@ __global__ void __launch_bounds__(tg::kThreads) k_conv3x3_tg(const bf16 *__restr
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const unsigned GW = (unsigned)(W + 7) / 8, groups = (unsigned)N * H * GW;
   const int tiles = (int)((groups + 15) / 16);
-  const uint32_t ncols = (uint32_t)tc::tmem_cols(2 * NC);
+  const uint32_t ncols = (uint32_t)tmem_cols(2 * NC);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::saddr(tslot)),
                  "r"(ncols)
@@ -563,7 +538,7 @@ __global__ void __launch_bounds__(kWgThreads) k_wgrad_tc(const bf16 *__restrict_
   const long long HW = (long long)H * W, P = (long long)N * HW;
   const long long pb = (long long)blockIdx.x * ppc, pe = min(P, pb + ppc);
   const int R = (int)((pe - pb + 16 * kWgRound - 1) / (16 * kWgRound));   // rounds
-  const uint32_t ncols = (uint32_t)tc::tmem_cols(NN);
+  const uint32_t ncols = (uint32_t)tmem_cols(NN);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::saddr(tslot)),
                  "r"(ncols)
@@ -1178,7 +1153,7 @@ __global__ void k_illum(float *__restrict__ illum, const float *__restrict__ p, 
 size_t conv_tc_smem(int cin, int cout) {
   const int T = tc::taps_per_round(cin, cout);
   const size_t need = (T == 9 ? 1 : 2) * (size_t)tc::stage_bytes(cin, cout, T) + 32;
-  const int fit = 512 / tc::tmem_cols(cout);   // CTAs whose accumulators fit
+  const int fit = 512 / tmem_cols(cout);   // CTAs whose accumulators fit
   if (fit >= 16) return need;                 // 16 CTAs of 128 threads fill an SM
   const size_t sm_bytes = 228 * 1024, reserve = 1024;   // per SM, per CTA
   const size_t cap = sm_bytes / (fit + 1) - reserve + 16;   // fit + 1 CTAs no longer fit
@@ -1217,7 +1192,7 @@ long long wgrad_pix_per_chunk(long long P, int cin) {
 
 size_t wgrad_tc_smem(int cin, int cout) {
   const size_t need = (size_t)wg_stages(cin, cout) * wg_stage_bytes(cin, cout) + 9 * 8 + 8;
-  const int fit = 512 / tc::tmem_cols(wg_cols(cin));   // CTAs whose accumulators fit
+  const int fit = 512 / tmem_cols(wg_cols(cin));   // CTAs whose accumulators fit
   const size_t cap = 228 * 1024 / (fit + 1) - 1024 + 16;   // fit + 1 CTAs no longer fit
   return std::max(need, cap);
 }
@@ -1271,13 +1246,6 @@ dim3 row_grid(int C, int rows, int W) {
 
 }  // namespace
 
-// Dynamic shared memory, raised where needed so that no more CTAs are
-// resident on an SM than its tensor memory holds.
-size_t conv_tg_smem(int cin, int cout) {
-  const int fit = 512 / tc::tmem_cols(2 * tg::cols(cin, cout));   // CTAs whose accumulators fit
-  return std::max(tg::smem(cin, cout), (size_t)(228 * 1024 / (fit + 1) - 1024 + 16));
-}
-
 template <bool F32, int KC>
 void conv_tg_kc(const bf16 *in, const bf16 *w, const float *bias, void *out, bool accum, int cout, int N, int H,
                 int W, cudaStream_t st) {
@@ -1288,7 +1256,7 @@ void conv_tg_kc(const bf16 *in, const bf16 *w, const float *bias, void *out, boo
   }();
   (void)attr;
   const long long tiles = ((long long)N * H * ((W + 7) / 8) + 15) / 16;
-  const size_t smem = conv_tg_smem(16 * KC, cout);
+  const size_t smem = tg::launch_smem(16 * KC, cout);
   const int halves = cout / tg::cols(16 * KC, cout);
   const long long ctas = std::max(1LL, (smem <= 112 * 1024 ? 296LL : 148LL) / halves);   // one or two an SM
   // tiles evenly over the CTAs
@@ -1318,9 +1286,9 @@ void launch_conv3x3(const bf16 *in, int cin, const bf16 *w, const float *bias, v
                 "conv widths must be multiples of 16, at most 128 in and 256 out");
   SWFWI_REQUIRE(N > 0 && H > 0 && W > 0, "conv image size out of range");
   SWFWI_REQUIRE(out_f32 || bias, "BF16 conv output needs a bias");
-  // row tiles (each input row staged once) where weights and two stages fit,
-  // and their group index 32 bits; else the pixel-run tiles
-  const bool rows = tg::stages(cin, cout) >= 2 && (long long)N * H * ((W + 7) / 8) < (1LL << 31) - 32;
+  // row tiles (each input row staged once) where weights, two stages and two
+  // accumulators fit, and their group index 32 bits; else the pixel-run tiles
+  const bool rows = tg::fits(cin, cout) && (long long)N * H * ((W + 7) / 8) < (1LL << 31) - 32;
   if (out_f32) {
     if (!(rows && conv_tg_go<true>(in, cin, w, bias, out, accum, cout, N, H, W, st)))
       conv_tc_go<true>(in, cin, w, bias, out, accum, cout, N, H, W, st);
