@@ -49,6 +49,14 @@ int guarded(F &&f) {
   }
 }
 
+// Lets a kernel's launches have `bytes` of dynamic shared memory.  The limit is
+// the current device's (and its context's) own, so launches that need it ask
+// each time; it takes a fraction of a microsecond.
+template <typename K>
+void allow_smem(K *kernel, size_t bytes) {
+  SWFWI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 // cudaMalloc; if the device is full, once more without this context's kept
 // scratch.
 void *device_alloc(size_t bytes);

@@ -735,13 +735,7 @@ void gain_on_device(const float *hona, const float *dobs, const double *z, long 
   } else {
     SWFWI_CUDA(cudaMemcpyAsync(sc.sigma, sigma_in, sizeof(double), cudaMemcpyHostToDevice, st));
   }
-  // once each (thread-safe static init)
-  static const cudaError_t attr_z = cudaFuncSetAttribute(k_cross<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)cross_smem_bytes());
-  static const cudaError_t attr_d = cudaFuncSetAttribute(k_cross<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)cross_smem_bytes());
-  SWFWI_CUDA(attr_z);
-  SWFWI_CUDA(attr_d);
+  allow_smem(z ? k_cross<false> : k_cross<true>, cross_smem_bytes());
   if (z)
     k_cross<false><<<nparts, kCrossThreads, cross_smem_bytes(), st>>>(sc.partials, hona, dobs, z, rows, n, sc.sigma,
                                                                       seed);
@@ -778,7 +772,7 @@ void fetch_gain(GainScratch &sc, int n, double *sigma, double *t4, int *clip, cu
 
 template <typename F, typename... Args>
 void launch_update(F kernel, long long model, cudaStream_t st, Args... args) {
-  SWFWI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem_bytes()));
+  allow_smem(kernel, update_smem_bytes());
   kernel<<<(unsigned)std::min<long long>((model + kTile - 1) / kTile, 444), kThreads, update_smem_bytes(), st>>>(
       args...);
   note_launch();

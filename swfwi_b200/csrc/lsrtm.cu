@@ -349,10 +349,7 @@ constexpr size_t kPrtmMaxSmem = 227 * 1024;
 
 template <int ARITH, int MODE>
 void prtm_resident_launch(const PrtmResident &a, size_t smem, cudaStream_t st) {
-  // raise the dynamic shared memory limit once (thread-safe static init)
-  static const cudaError_t attr = cudaFuncSetAttribute(k_prtm_resident<ARITH, MODE>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrtmMaxSmem);
-  SWFWI_CUDA(attr);
+  allow_smem(k_prtm_resident<ARITH, MODE>, kPrtmMaxSmem);
   PrtmResident b = a;
   void *args[] = {&b};
   SWFWI_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_prtm_resident<ARITH, MODE>),

@@ -12,13 +12,10 @@ namespace {
 constexpr size_t kMaxSmem = 227 * 1024;
 
 int device_sms() {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    SWFWI_CUDA(cudaGetDevice(&dev));
-    SWFWI_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-    return n;
-  }();
-  return sms;
+  int dev = 0, n = 0;
+  SWFWI_CUDA(cudaGetDevice(&dev));
+  SWFWI_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+  return n;
 }
 
 int depth_groups(int nz) { return (nz - 6) / 4 + ((nz - 6) % 4 == 3 ? 1 : 0); }
@@ -79,10 +76,7 @@ int row_chunks(bool back, int rmax, int ngroups, int warps) {
 
 template <int ARITH, bool BACK, bool WIDE>
 void launch_t(const ResidentArgs &a, size_t smem, cudaStream_t st) {
-  // raise the dynamic shared memory limit once (thread-safe static init)
-  static const cudaError_t attr = cudaFuncSetAttribute(fd_resident<ARITH, BACK, WIDE>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-  SWFWI_CUDA(attr);
+  allow_smem(fd_resident<ARITH, BACK, WIDE>, kMaxSmem);
   ResidentArgs b = a;
   void *args[] = {&b};
   SWFWI_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fd_resident<ARITH, BACK, WIDE>),
