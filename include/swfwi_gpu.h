@@ -152,6 +152,16 @@ int swfwi_damp4t10d_set_fusion(swfwi_damp4t10d *h, int on);
  * propagator's stream (one graph per loop and setting, stencil timing
  * included).  Same kernels, same results. */
 int swfwi_damp4t10d_set_graphs(swfwi_damp4t10d *h, int on);
+/* cycles that a sweep with its fields on chip may wait for a neighbour's rows
+ * before it gives up (default 2^31, about a second; 0: one unsuccessful
+ * poll).  A sweep that gave up leaves NaN in the records and images it had
+ * not written. */
+int swfwi_damp4t10d_set_wait_limit(swfwi_damp4t10d *h, long long cycles);
+/* Waits for the propagator's stream and reports SWFWI_ERR_TIMEOUT, once, if
+ * a kernel's bounded wait gave up since the last report.  Calls that return
+ * results to the host (objectives, member batches, epochs) do so themselves;
+ * the asynchronous ones (modelling, calgradient) leave it to this. */
+int swfwi_damp4t10d_check(swfwi_damp4t10d *h);
 /* Per-shot receiver lists (uneven spreads; not in the reference, whose
  * ShotPosition is one common line): shot s has receivers
  * [offsets[s], offsets[s+1]) of gx/gz (unpadded, host arrays).  The
@@ -364,6 +374,13 @@ int swfwi_prtm2d_set_graphs(swfwi_prtm *h, int on);
 /* on = 1 (default): sweeps run as one launch with their fields on chip where
  * the grid allows it; 0: as the launched time loops (set_graphs). */
 int swfwi_prtm2d_set_resident(swfwi_prtm *h, int on);
+/* cycles that an on-chip sweep may wait for a neighbour's rows before it
+ * gives up (default 2^31, about a second; 0: one unsuccessful poll).  A sweep
+ * that gave up leaves NaN in what it had not written; the next lop, or
+ * swfwi_prtm2d_check, reports SWFWI_ERR_TIMEOUT once. */
+int swfwi_prtm2d_set_wait_limit(swfwi_prtm *h, long long cycles);
+/* waits for stream and reports a sweep that gave up since the last report */
+int swfwi_prtm2d_check(swfwi_prtm *h, void *stream);
 /* shots one launch sequence carries (1 for REF) */
 int swfwi_prtm2d_batch(swfwi_prtm *h, int *shots);
 /* prtm2d_lop (:354-437): adj = 0: dat += L mod (Born); adj = 1: mod += L'

@@ -102,6 +102,8 @@ _SIGS = {
     "swfwi_fwi_set_velocity": [_vp, _fp],
     "swfwi_damp4t10d_set_fusion": [_vp, C.c_int],
     "swfwi_damp4t10d_set_graphs": [_vp, C.c_int],
+    "swfwi_damp4t10d_set_wait_limit": [_vp, C.c_longlong],
+    "swfwi_damp4t10d_check": [_vp],
     "swfwi_rsf_get": [C.c_char_p, C.c_char_p, C.c_char_p, C.c_int],
     "swfwi_rsf_dims": [C.c_char_p, _ip, _ip, _fp, _fp],
     "swfwi_rsf_read": [C.c_char_p, _fp, C.c_longlong, C.c_longlong],
@@ -153,6 +155,8 @@ _SIGS = {
     "swfwi_prtm2d_set_adjoint": [_vp, C.c_int],
     "swfwi_prtm2d_set_graphs": [_vp, C.c_int],
     "swfwi_prtm2d_set_resident": [_vp, C.c_int],
+    "swfwi_prtm2d_set_wait_limit": [_vp, C.c_longlong],
+    "swfwi_prtm2d_check": [_vp, _vp],
     "swfwi_prtm2d_batch": [_vp, _ip],
     "swfwi_prtm2d_lop": [_vp, C.c_int, C.c_int, C.c_int, C.c_int, _vp, _vp, _vp],
     "swfwi_prtm2d_destroy": [_vp],
@@ -484,6 +488,16 @@ class Prtm2d:
         or always as launched time loops."""
         _check(lib().swfwi_prtm2d_set_resident(self.h, int(bool(on))))
 
+    def set_wait_limit(self, cycles: int) -> None:
+        """Cycles that an on-chip sweep may wait for a neighbour's rows before
+        it gives up and leaves NaN in what it had not written."""
+        _check(lib().swfwi_prtm2d_set_wait_limit(self.h, cycles))
+
+    def check(self, stream=None) -> None:
+        """Waits for the stream; raises SwfwiError (timeout) if a sweep gave
+        up since the last report.  The next ``lop`` raises it as well."""
+        _check(lib().swfwi_prtm2d_check(self.h, _stream(stream)))
+
     def batch(self) -> int:
         out = C.c_int()
         _check(lib().swfwi_prtm2d_batch(self.h, C.byref(out)))
@@ -590,6 +604,18 @@ class Damp4t10d:
         """CUDA graphs for the forward/backward time loops: False/0 never,
         True/1 for small (launch-bound) steps, 2 for every step size."""
         _check(lib().swfwi_damp4t10d_set_graphs(self.h, int(on)))
+
+    def set_wait_limit(self, cycles: int):
+        """Cycles that a sweep with its fields on chip may wait for a
+        neighbour's rows before it gives up and leaves NaN in its results."""
+        _check(lib().swfwi_damp4t10d_set_wait_limit(self.h, cycles))
+
+    def check(self):
+        """Waits for the stream; raises SwfwiError (timeout) if a kernel's
+        bounded wait gave up since the last report.  For the asynchronous
+        calls (modelling, calgradient); those that return objectives check
+        themselves."""
+        _check(lib().swfwi_damp4t10d_check(self.h))
 
     def set_strip_format(self, fmt: int):
         """Boundary strips of the gradients: STRIP_F32 (exact), STRIP_F16 or

@@ -227,6 +227,17 @@ int swfwi_damp4t10d_set_graphs(swfwi_damp4t10d *h, int on) {
   });
 }
 
+int swfwi_damp4t10d_set_wait_limit(swfwi_damp4t10d *h, long long cycles) {
+  return guarded([&] {
+    SWFWI_REQUIRE(cycles >= 0, "negative wait limit");
+    P(h).wait_limit = cycles;
+  });
+}
+
+int swfwi_damp4t10d_check(swfwi_damp4t10d *h) {
+  return guarded([&] { P(h).check_device_error(); });
+}
+
 int swfwi_damp4t10d_set_tuning(swfwi_damp4t10d *h, int kernel, int band_depth, int rows_per_cta,
                                int rows_in_flight, int shots_slowest) {
   return guarded([&] {

@@ -450,7 +450,7 @@ void Propagator::check_device_error() {
   SWFWI_CUDA(cudaStreamSynchronize(st_));
   if (e) {
     SWFWI_CUDA(cudaMemsetAsync(d_err_.get(), 0, sizeof(int), st_));
-    throw Error(SWFWI_ERR_TIMEOUT, "a stencil kernel's bounded wait on its row pipeline gave up");
+    throw Error(SWFWI_ERR_TIMEOUT, "a stencil kernel's bounded wait gave up (on its row pipeline or a neighbour's rows)");
   }
 }
 
@@ -798,6 +798,7 @@ bool Propagator::resident_forward(Work<float> &w, int n, PointSet src, const flo
     a.dt = dt;
     a.halo = res_halo_.get();
     a.err = d_err_.get();
+    a.patience = wait_limit;
     launch_resident(arith, false, p, a, std::min(p.slots, n - s0), st_);
   }
   return true;
@@ -856,6 +857,7 @@ bool Propagator::resident_backward(Work<float> &w, int n, PointSet src, const fl
     a.dt = dt;
     a.halo = res_halo_.get();
     a.err = d_err_.get();
+    a.patience = wait_limit;
     launch_resident(arith, true, p, a, std::min(p.slots, n - s0), st_);
   }
   return true;

@@ -126,6 +126,9 @@ class Propagator {
   int stream_depth = 3;       // rows ahead (3 or 7)
   int stream_shot_major = 0;  // launch order: 0 = shots fastest
   bool fuse = false;          // fused time loops where they apply
+  // Cycles that a resident sweep's wait on its neighbours may take before it
+  // gives up; 0: one unsuccessful poll.
+  long long wait_limit = 1LL << 31;
   // Source illumination: while set, the forward sweeps that save strips
   // add sum over slots of p^2 into illum [nxpad][nzpad] every illum_every
   // steps (the caller zeroes it).

@@ -448,10 +448,9 @@ class Prtm {
       }
     }
     geo_serial_ = ng > 1 && jgx == 0 && jgz == 0;
-    err_.resize(1);
-    err_.zero(st);
-    SWFWI_CUDA(cudaHostAlloc(&h_err_, sizeof(int), cudaHostAllocDefault));
-    *h_err_ = 0;
+    // written by a sweep that gives up, read by the host without a copy
+    SWFWI_CUDA(cudaHostAlloc(&err_, sizeof(int), cudaHostAllocMapped));
+    *err_ = 0;
     int dev = 0;
     SWFWI_CUDA(cudaGetDevice(&dev));
     SWFWI_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
@@ -461,7 +460,7 @@ class Prtm {
   }
 
   ~Prtm() {
-    if (h_err_) cudaFreeHost(h_err_);
+    if (err_) cudaFreeHost(err_);   // waits for the sweeps in flight
     for (Graph &g : graphs_)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     if (cap_) cudaStreamDestroy(cap_);
@@ -479,6 +478,15 @@ class Prtm {
   }
   void set_graphs(bool on) { use_graphs_ = on; }
   void set_resident(bool on) { use_resident_ = on; }
+  void set_wait_limit(long long cycles) {
+    SWFWI_REQUIRE(cycles >= 0, "negative wait limit");
+    wait_limit_ = cycles;
+  }
+  // Waits for st and reports a wait that gave up in any call since the last report.
+  void check(cudaStream_t st) {
+    SWFWI_CUDA(cudaStreamSynchronize(st));
+    report();
+  }
 
   // prtm2d_lop (:354-437) on device arrays.  A call that repeats an earlier
   // one's arrays, direction and mode replays the time loops as one CUDA
@@ -495,11 +503,7 @@ class Prtm {
       }
       for (int s0 = 0; s0 < ns_; s0 += kmax_) run(adj, mod, dat, s0, std::min(kmax_, ns_ - s0), s);
     };
-    if (*h_err_) {   // as far as earlier calls are known to have finished
-      *h_err_ = 0;
-      err_.zero(st);
-      throw Error(SWFWI_ERR_TIMEOUT, "a resident sweep's bounded wait on its neighbours gave up");
-    }
+    report();   // as far as earlier calls have got
     // resident sweeps are a launch or two each: nothing for a graph to gain
     if (!use_graphs_ || resident(adj)) {
       body(st);
@@ -557,6 +561,12 @@ class Prtm {
   static constexpr size_t kGraphs = 4;
 
   // ---- resident sweeps ----
+  void report() {
+    if (!*static_cast<volatile int *>(err_)) return;
+    SWFWI_CUDA(cudaDeviceSynchronize());   // the sweep's other blocks have raised it too
+    *static_cast<volatile int *>(err_) = 0;
+    throw Error(SWFWI_ERR_TIMEOUT, "a resident sweep's bounded wait on its neighbours gave up");
+  }
   PrtmPlan plan_resident_sweep(int mode) const {
     PrtmPlan p;
     // injection at one shared cell has an order; a one-step sweep exchanges
@@ -587,7 +597,7 @@ class Prtm {
     p.slots = (kmax_ + rounds - 1) / rounds;
     p.cps = std::min(most, sms_ / p.slots);
     need(p.cps);
-    p.halo = (size_t)p.slots * p.cps * (mode == PRTM_SOURCE ? 1 : 2) * 4 * 4 * p.ogroups;
+    p.halo = (size_t)p.slots * p.cps * (mode == PRTM_SOURCE ? 1 : 2) * 4 * 4 * p.ogroups + 1;   // and the launch's flag
     // row chunks: about 170 instructions an output row of both pairs, 14 a
     // row to fill the queue; a round of warps as in the propagator's sweeps
     const int warps = kPrtmThreads / 32 - kPrtmHelpers;
@@ -648,7 +658,9 @@ class Prtm {
       a.img = img ? img + c * img_stride : nullptr;
       a.img_stride = img_stride;
       a.halo = halo_.get();
-      a.err = err_.get();
+      a.quit = reinterpret_cast<int *>(a.halo + p.halo - 1);
+      a.err = err_;
+      a.patience = wait_limit_;
       SWFWI_CUDA(cudaMemsetAsync(halo_.get(), 0, sizeof(uint4) * p.halo, st));
       if (arith_ == ARITH_REF) prtm_resident_mode<ARITH_REF>(mode, a, p.smem, st);
       else prtm_resident_mode<ARITH_FAST>(mode, a, p.smem, st);
@@ -693,7 +705,6 @@ class Prtm {
         SWFWI_CUDA(cudaMemsetAsync(G1, 0, fbytes, st));
       }
     }
-    SWFWI_CUDA(cudaMemcpyAsync(h_err_, err_.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
   }
 
   int pidx(int x, int z) const { return (x + nb_) * nzpad_ + z + nb_; }
@@ -894,8 +905,8 @@ class Prtm {
   PrtmPlan plan_[4];               // by PrtmSweep
   std::vector<int> row_rec_;
   DevBuf<uint4> halo_;
-  DevBuf<int> err_;
-  int *h_err_ = nullptr;
+  int *err_ = nullptr;             // mapped host memory
+  long long wait_limit_ = 1LL << 31;
   PrtmCoef c_{};
   PrtmGeo geo_{};
   DevBuf<float> vv_, wlt_, sponge_, sp0_, sp1_, gp0_, gp1_, gp2_, ring_, img_;
@@ -944,6 +955,20 @@ extern "C" int swfwi_prtm2d_set_resident(swfwi_prtm *h, int on) {
   return guarded([&] {
     SWFWI_REQUIRE(h && h->p, "null handle");
     h->p->set_resident(on != 0);
+  });
+}
+
+extern "C" int swfwi_prtm2d_set_wait_limit(swfwi_prtm *h, long long cycles) {
+  return guarded([&] {
+    SWFWI_REQUIRE(h && h->p, "null handle");
+    h->p->set_wait_limit(cycles);
+  });
+}
+
+extern "C" int swfwi_prtm2d_check(swfwi_prtm *h, void *stream) {
+  return guarded([&] {
+    SWFWI_REQUIRE(h && h->p, "null handle");
+    h->p->check(reinterpret_cast<cudaStream_t>(stream));
   });
 }
 

@@ -46,7 +46,8 @@ struct PrtmResident {
   float *dat, *ring, *img;
   long long ring_stride, img_stride;
   uint4 *halo;                 // zeroed before the launch
-  int *err;
+  int *quit, *err;             // a wait gave up: the launch's flag (zeroed before it), the caller's
+  long long patience;          // cycles a wait may take; 0: one unsuccessful poll
 };
 
 struct PrtmSlab {
@@ -205,18 +206,46 @@ __device__ __noinline__ void prtm_receive(const PrtmResident &a, float *F, int c
       if (x.y == tag && x.w == tag && y.y == tag && y.w == tag) {
         st4(to, make_float4(__uint_as_float(x.x), __uint_as_float(x.z), __uint_as_float(y.x), __uint_as_float(y.z)));
         todo = false;
-      } else if ((spin & 255) == 255) {
-        // bounded: about a second, or until another CTA gave up
+      } else if (a.patience == 0 || (spin & 255) == 255) {
+        // bounded: a.patience cycles, or until another CTA gave up
         const long long now = clock64();
         if (t0 == 0) t0 = now;
-        if (now - t0 > (1LL << 31) || *(volatile int *)a.err) {
-          atomicExch(a.err, 1);
+        if (now - t0 >= a.patience || *(volatile int *)a.quit) {
+          *(volatile int *)a.quit = 1;
+          *(volatile int *)a.err = 1;
           b.give_up = 1;
           break;
         }
       }
     }
     __syncwarp();
+  }
+}
+
+// A wait gave up in step n: what the CTA would still have written is NaN, the
+// data from the next step on, the source pair or the image.
+template <int MODE>
+__device__ __noinline__ void prtm_spoil(const PrtmResident &a, float *F, int n) {
+  const PrtmLayout l(MODE, a.rmax, a.zp, a.cap_rec, a.cap_ring);
+  const PrtmSlab &b = *reinterpret_cast<const PrtmSlab *>(F + l.slab);
+  const int tid = threadIdx.x, nthreads = blockDim.x, nzp = a.g.nzpad, nb = a.g.nb;
+  const float nan = __int_as_float(0x7fffffff);
+  if constexpr (MODE == PRTM_BORN) {
+    const int *idx = reinterpret_cast<const int *>(F + l.rec) + a.cap_rec;
+    for (int k = 0; k < b.nrec; k++)
+      for (int it = n + 1 + tid; it < a.g.nt; it += nthreads)
+        a.dat[((long long)b.slot * a.g.ng + idx[k]) * a.g.nt + it] = nan;
+  } else {
+    for (int i = tid; i < b.R * nzp; i += nthreads) {
+      const int r = i / nzp, z = i - r * nzp, mx = b.xa + r - nb, mz = z - nb;
+      if constexpr (MODE == PRTM_SOURCE) {
+        const long long p = (long long)b.slot * a.g.fsz + (long long)(b.xa + r) * nzp + z;
+        if (z >= 2 && z < nzp - 2) a.s0[p] = a.s1[p] = nan;
+      } else {
+        if (mx >= 0 && mx < a.g.nx && mz >= 0 && mz < a.g.nz)
+          a.img[(long long)b.slot * a.img_stride + (long long)mx * a.g.nz + mz] = nan;
+      }
+    }
   }
 }
 
@@ -563,7 +592,10 @@ __global__ void __launch_bounds__(kPrtmThreads, 1) k_prtm_resident(const __grid_
     if constexpr (BACKW) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     cur ^= 1;
-    if (sb.give_up) return;   // uniform: written before the barrier, never cleared
+    if (sb.give_up) {   // uniform: written before the barrier, never cleared
+      prtm_spoil<MODE>(sa, F, n);
+      return;
+    }
   }
 
   // ---- results

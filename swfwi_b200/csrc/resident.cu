@@ -140,7 +140,7 @@ static ResidentPlan plan_slabs(bool thin, int arith, bool back, int n, int nx, i
   p.helpers = 3;
   p.chunks = row_chunks(back, p.rmax, p.ngroups, kResidentThreads / 32 - p.helpers);
   if (resident_halo(p.slots, p.cps, rows, p.thin, 2, p.ogroups) >= (1u << 31)) return ResidentPlan();
-  p.halo = resident_halo(p.slots, p.cps, rows, p.thin, back ? 2 : 1, p.ogroups);
+  p.halo = resident_halo(p.slots, p.cps, rows, p.thin, back ? 2 : 1, p.ogroups) + 1;   // and the launch's flag
   p.ok = true;
   return p;
 }
@@ -199,7 +199,8 @@ void launch_resident(int arith, bool back, const ResidentPlan &p, ResidentArgs a
   a.cap_rec = p.cap_rec;
   a.cap_stage = p.cap_stage;
   const size_t halo = resident_halo(nslots, p.cps, p.rows, p.thin, back ? 2 : 1, p.ogroups);
-  SWFWI_CUDA(cudaMemsetAsync(a.halo, 0, sizeof(uint4) * halo, st));
+  a.quit = reinterpret_cast<int *>(a.halo + halo);
+  SWFWI_CUDA(cudaMemsetAsync(a.halo, 0, sizeof(uint4) * (halo + 1), st));
   auto go = [&](auto wide) {
     constexpr bool W = decltype(wide)::value;
     if (arith == ARITH_REF) {

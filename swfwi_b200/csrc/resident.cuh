@@ -45,7 +45,9 @@
 // buffer then has a place for every row, read by whoever is within 6 of it;
 // who reads a CTA's rows is again who it reads.  Every CTA of the grid is
 // resident (cooperative launch), every wait is bounded: on timeout the CTA
-// raises the error flag, which the others' waits look at, and leaves.
+// raises the launch's flag, which the others' waits look at, and the
+// caller's, which stays up until the host has seen it; it makes its results
+// NaN, so that they cannot pass for a sweep's, and leaves.
 #pragma once
 #include <type_traits>
 #include "kernels.cuh"
@@ -89,7 +91,9 @@ struct ResidentArgs {
   unsigned nzs_magic;        // 2^32 / nzs + 1: u / nzs = high word of u * nzs_magic, nzs = depths of a side strip
   int thin;                  // slabs of fewer than 6 rows (two-pass form only): exchange buffer by row, not by slab
   uint4 *halo;               // zeroed before the launch
-  int *err;
+  int *quit;                 // this launch's flag: a wait gave up (zeroed before the launch)
+  int *err;                  // the caller's
+  long long patience;        // cycles a wait may take; 0: one unsuccessful poll
 };
 
 constexpr int kResidentThreads = 512;
@@ -329,12 +333,13 @@ __device__ __noinline__ void receive_step(const ResidentArgs &a, float *F, int c
       }
     }
     long long t0 = 0;
-    auto late = [&](int spin) {   // bounded: about a second, or until another CTA gave up
-      if ((spin & 255) != 255) return false;
+    auto late = [&](int spin) {   // bounded: a.patience cycles, or until another CTA gave up
+      if (a.patience > 0 && (spin & 255) != 255) return false;
       const long long now = clock64();
       if (t0 == 0) t0 = now;
-      if (now - t0 <= (1LL << 31) && !*(volatile int *)a.err) return false;
-      atomicExch(a.err, 1);
+      if (now - t0 < a.patience && !*(volatile int *)a.quit) return false;
+      *(volatile int *)a.quit = 1;
+      *(volatile int *)a.err = 1;
       b.give_up = 1;
       return true;
     };
@@ -357,6 +362,30 @@ __device__ __noinline__ void receive_step(const ResidentArgs &a, float *F, int c
     }
     __syncwarp();
   }
+}
+
+// A wait gave up in step n: what the CTA would still have written is NaN, the
+// records from the next step on and the final pair, or the image.
+template <bool BACK>
+__device__ __noinline__ void spoil_results(const ResidentArgs &a, float *F, int n) {
+  const ResidentLayout l(BACK, a.rmax, a.zp, a.cap_src, a.cap_rec, a.cap_stage);
+  const ResidentSlab &b = *reinterpret_cast<const ResidentSlab *>(F + l.slab);
+  const int tid = threadIdx.x, nthreads = blockDim.x;
+  const float nan = __int_as_float(0x7fffffff);
+  if (!BACK && a.dcal) {
+    const int *rec_idx = reinterpret_cast<const int *>(F + l.rec) + a.cap_rec;
+    for (int it = n + 1; it < a.steps; it++)
+      for (int k = tid; k < b.nrec; k += nthreads)
+        a.dcal[((long long)b.slot * a.nt + it) * a.ngrec + rec_idx[k]] = nan;
+  }
+  if (BACK || a.store_state)
+    for (int i = tid; i < b.R * a.zp; i += nthreads) {
+      const int r = i / a.zp, z = i - r * a.zp;
+      if (z < 6 || z >= a.nz - 6) continue;
+      const long long p = (long long)b.slot * a.fstride + (long long)(b.xa + r) * a.pitch + z;
+      if constexpr (BACK) a.image[p] = nan;
+      else a.p0[p] = a.p1[p] = nan;
+    }
 }
 
 // The compute warps' part of a step in two passes (ct of cn threads).
@@ -852,7 +881,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1) fd_resident(const __grid_
     if constexpr (BACK) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     cur ^= 1;
-    if (sb.give_up) return;   // uniform: written before the barrier, never cleared
+    if (sb.give_up) {   // uniform: written before the barrier, never cleared
+      spoil_results<BACK>(sa, F, n);
+      return;
+    }
   }
 
   // ---- results
