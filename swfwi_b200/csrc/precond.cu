@@ -437,7 +437,8 @@ __global__ void __launch_bounds__(tg::kThreads) k_conv3x3_tg(const bf16 *__restr
       const long long p = valid ? (long long)row * W + x : 0;
       const bool got = mbar_wait(&ready[buf], (uint32_t)((k / 2) & 1));
       if (!got) *bad = 1;
-      if (!__all_sync(0xffffffffu, got) || *bad) break;
+      // one decision a warp: the reads of tensor memory are whole warps'
+      if (__any_sync(0xffffffffu, !got || *bad)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       for (int c0 = 0; c0 < NC; c0 += 16) {
         uint32_t v[16];

@@ -53,3 +53,14 @@ def test_the_networks_layers_take_row_tiles(shapes):
     for cin, cout in ((16, 16), (16, 32), (32, 32), (32, 64), (64, 64), (128, 64), (96, 32), (48, 16),
                       (16, 48), (32, 96), (64, 128), (32, 16), (64, 32)):
         assert (cin, cout) in taken, (cin, cout)
+
+
+def test_epilogue_leaves_by_a_vote():
+    """Reads of tensor memory need whole warps: where the row-tile kernel's
+    epilogue may leave its loop on a wait that gave up, the warp votes."""
+    with open(os.path.join(ROOT, "swfwi_b200", "csrc", "precond.cu")) as f:
+        text = f.read()
+    at = text.index("// ---- epilogue")
+    loop = text[at:text.index("tcgen05.ld.sync", at)]
+    leaves = [line.strip() for line in loop.splitlines() if "break;" in line]
+    assert leaves and all(line.startswith("if (__any_sync(0xffffffffu,") for line in leaves), leaves
