@@ -454,7 +454,12 @@ class Prtm {
     int dev = 0;
     SWFWI_CUDA(cudaGetDevice(&dev));
     SWFWI_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
-    for (int m = 0; m < 4; m++) plan_[m] = plan_resident_sweep(m);
+    size_t halo = 0;   // one buffer for every sweep: a call allocates nothing
+    for (int m = 0; m < 4; m++) {
+      plan_[m] = plan_resident_sweep(m);
+      if (plan_[m].ok) halo = std::max(halo, plan_[m].halo);
+    }
+    halo_.resize(halo);
     geo_ = PrtmGeo{nx, nz, nb, nxpad_, nzpad_, nt, ng, (long long)fsz, spos_.get(), rpos_.get(), sponge_.get(),
                    ng > 1 && jgx == 0 && jgz == 0 ? 1 : 0};
   }
@@ -625,7 +630,6 @@ class Prtm {
   void resident_sweep(int mode, float *mod, float *dat, float *img, long long img_stride, float *G0, float *G1, int s0,
                       int k, cudaStream_t st) {
     const PrtmPlan &p = plan_[mode];
-    halo_.resize(p.halo);
     for (int c = 0; c < k; c += p.slots) {
       PrtmResident a{};
       a.g = geo_;
