@@ -135,7 +135,8 @@ int swfwi_damp4t10d_set_reconstruction(swfwi_damp4t10d *h, int mode, int every, 
  * task (at least 8 rows) with which every (shot, depth slice) column's
  * tasks fit in one wave of resident warps, kernel 1 takes 64;
  * shots_slowest = 1 runs the CTAs of one
- * shot together (kernel 1). */
+ * shot together (kernel 1).  Kernel 6 with rows per CTA 0 also lets small
+ * sweeps run in one launch with their fields on chip; other shapes stream. */
 int swfwi_damp4t10d_set_tuning(swfwi_damp4t10d *h, int kernel, int band_depth, int rows_per_cta,
                                int rows_in_flight, int shots_slowest);
 /* Fused backward time loop (default off): where sources and receivers form
@@ -414,7 +415,9 @@ int swfwi_fwi_last_trials(const swfwi_fwi *h, int *trials);
  * replay; its timed stencil launches are bracketed by event nodes in the
  * graph, their times added after each replay completes.
  * step_ms is the timed launches' total: their mean is step_ms /
- * step_timed_launches.
+ * step_timed_launches.  A sweep that runs in one launch counts as its steps'
+ * launches (two a step going backward), timed as a whole.  Timing changes
+ * neither the kernels that run nor their results.
  * ---------------------------------------------------------------------- */
 typedef struct {
   long long kernel_launches;

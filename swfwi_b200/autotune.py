@@ -9,6 +9,11 @@ wave of tasks), rows in flight ahead of the compute and the launch
 order (shots slowest or fastest).  ``tune`` times short batched forward runs of a survey for each
 candidate with the library's CUDA-event step timing and returns the fastest;
 ``apply`` sets it on a propagator.
+
+Only kernel 6 with the automatic length leaves the choice between streaming
+and one launch a sweep with the fields on chip (``resident.cuh``) to the
+propagator; every other shape streams.  The timing covers either form, so a
+survey that is faster on chip keeps it.
 """
 from __future__ import annotations
 

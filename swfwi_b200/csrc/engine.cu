@@ -64,16 +64,17 @@ void StepTimer::read(double &ms, long long &n, double &pts, double &b, long long
   for (Capture *c : replayed) harvest(c);
   replayed.clear();
   ms = graph_ms;
+  timed = graph_timed;
   for (size_t i = 0; i < used; i++) {
     SWFWI_CUDA(cudaEventSynchronize(pool[i].second));
     float t = 0;
     SWFWI_CUDA(cudaEventElapsedTime(&t, pool[i].first, pool[i].second));
-    ms += t;
+    ms += pool[i].steps == 1 ? t : t * (double)pool[i].timed / pool[i].steps;
+    timed += pool[i].timed;
   }
   n = launches;
   pts = points;
   b = bytes;
-  timed = (long long)used + graph_timed;
 }
 
 // Algorithmic work of one step launch: every interior point of every field
@@ -81,16 +82,18 @@ void StepTimer::read(double &ms, long long &n, double &pts, double &b, long long
 // velocity model the launch uses is read once.  Inside a capture the work
 // goes to the capture (added per replay) and a timed launch gets its own
 // event pair, recorded as graph nodes.
-cudaEvent_t StepTimer::open(cudaStream_t st, double pts, int n, int nvel, int el) {
+cudaEvent_t StepTimer::open(cudaStream_t st, double pts, int n, int nvel, int el, long long steps) {
   if (!enabled.load(std::memory_order_relaxed)) return nullptr;
   std::lock_guard<std::mutex> g(mu);
   Capture *c = t_capturing;
-  const long long k = c ? c->launches++ : launches++;
-  (c ? c->points : points) += pts * n;
-  (c ? c->bytes : bytes) += pts * n * 3 * el + pts * el * nvel;
+  const long long k = c ? c->launches : launches;
+  (c ? c->launches : launches) += steps;
+  (c ? c->points : points) += pts * n * steps;
+  (c ? c->bytes : bytes) += (pts * n * 3 * el + pts * el * nvel) * steps;
   const int per = std::max(period.load(std::memory_order_relaxed), 1);
-  if (k % per != 0) return nullptr;
-  if (c) {
+  const long long due = (k + steps + per - 1) / per - (k + per - 1) / per;   // multiples of per in [k, k + steps)
+  if (due == 0) return nullptr;
+  if (c) {   // a captured loop launches its steps one by one
     cudaEvent_t x, y;
     SWFWI_CUDA(cudaEventCreate(&x));
     SWFWI_CUDA(cudaEventCreate(&y));
@@ -102,9 +105,11 @@ cudaEvent_t StepTimer::open(cudaStream_t st, double pts, int n, int nvel, int el
     cudaEvent_t x, y;
     SWFWI_CUDA(cudaEventCreate(&x));
     SWFWI_CUDA(cudaEventCreate(&y));
-    pool.emplace_back(x, y);
+    pool.push_back({x, y, 1, 1});
   }
-  auto ev = pool[used++];
+  Timed &ev = pool[used++];
+  ev.steps = steps;
+  ev.timed = due;
   SWFWI_CUDA(cudaEventRecord(ev.first, st));
   return ev.second;
 }
@@ -739,9 +744,8 @@ void Propagator::restore_snapshot(Work<T> &w, int n, int m, T *a, T *b) {
 
 // ---- resident time loops (resident.cuh) ----------------------------------
 bool Propagator::resident_allowed() const {
-  // the streaming kernels serve explicit launch shapes, fused loops and
-  // launches being timed
-  return stream_kernel == 6 && stream_xchunk <= 0 && !fuse && !step_timer().enabled.load(std::memory_order_relaxed);
+  // the streaming kernels serve explicit launch shapes and fused loops
+  return stream_kernel == 6 && stream_xchunk <= 0 && !fuse;
 }
 
 // The faster one by estimate; a resident sweep has to be clearly so, since
@@ -799,7 +803,11 @@ bool Propagator::resident_forward(Work<float> &w, int n, PointSet src, const flo
     a.halo = res_halo_.get();
     a.err = d_err_.get();
     a.patience = wait_limit;
-    launch_resident(arith, false, p, a, std::min(p.slots, n - s0), st_);
+    const int k = std::min(p.slots, n - s0);
+    cudaEvent_t done =
+        step_timer().open(st_, (double)(nxpad - 12) * (nzpad - 12), k, vel_stride_ ? k : 1, 4, a.steps);
+    launch_resident(arith, false, p, a, k, st_);
+    step_timer().close(done, st_);
   }
   return true;
 }
@@ -858,7 +866,11 @@ bool Propagator::resident_backward(Work<float> &w, int n, PointSet src, const fl
     a.halo = res_halo_.get();
     a.err = d_err_.get();
     a.patience = wait_limit;
-    launch_resident(arith, true, p, a, std::min(p.slots, n - s0), st_);
+    const int k = std::min(p.slots, n - s0);
+    cudaEvent_t done =
+        step_timer().open(st_, (double)(nxpad - 12) * (nzpad - 12), k, vel_stride_ ? k : 1, 4, 2LL * a.steps);
+    launch_resident(arith, true, p, a, k, st_);
+    step_timer().close(done, st_);
   }
   return true;
 }

@@ -24,6 +24,7 @@ namespace swfwi {
 // Process-wide timing of stencil launches (CUDA events on the launching
 // stream) and their algorithmic work, read by benchmarks.  While enabled,
 // every launch's work is counted and every period-th launch is timed.
+// Measuring changes neither the kernels that run nor their results.
 struct StepTimer {
   // What a captured time loop contributes each time its graph is replayed:
   // its stencil launches' count and work, its kernel launches, and the
@@ -39,7 +40,12 @@ struct StepTimer {
   std::atomic<bool> enabled{false};
   std::atomic<int> period{1};
   std::mutex mu;
-  std::vector<std::pair<cudaEvent_t, cudaEvent_t>> pool;
+  // of a sweep in one launch: its steps, and how many of them are timed
+  struct Timed {
+    cudaEvent_t first, second;
+    long long steps, timed;
+  };
+  std::vector<Timed> pool;
   size_t used = 0;
   long long launches = 0;
   double points = 0, bytes = 0;
@@ -51,8 +57,10 @@ struct StepTimer {
   void read(double &ms, long long &n, double &pts, double &b, long long &timed);
   // Opens the timing of one launch over n fields of pts interior points
   // reading nvel velocity models, el bytes an element; returns the event to
-  // record after the launch with close() (null when timing is off).
-  cudaEvent_t open(cudaStream_t st, double pts, int n, int nvel, int el);
+  // record after the launch with close() (null when timing is off).  A launch
+  // that runs a whole sweep counts as `steps` launches; it is timed if any of
+  // them would be, each with the mean.
+  cudaEvent_t open(cudaStream_t st, double pts, int n, int nvel, int el, long long steps = 1);
   void close(cudaEvent_t done, cudaStream_t st);
   // Stream capture of a time loop begins / ends (the kernels the capture
   // counted are taken back; each replay adds them).
