@@ -373,7 +373,8 @@ int swfwi_prtm2d_set_adjoint(swfwi_prtm *h, int mode);
  * the second such call); 0: every call launches its kernels one by one. */
 int swfwi_prtm2d_set_graphs(swfwi_prtm *h, int on);
 /* on = 1 (default): sweeps run as one launch with their fields on chip where
- * the grid allows it; 0: as the launched time loops (set_graphs). */
+ * the grid allows it and that is estimated to be faster; 0: as the launched
+ * time loops (set_graphs). */
 int swfwi_prtm2d_set_resident(swfwi_prtm *h, int on);
 /* cycles that an on-chip sweep may wait for a neighbour's rows before it
  * gives up (default 2^31, about a second; 0: one unsuccessful poll).  A sweep

@@ -341,7 +341,8 @@ namespace {
 // How a resident sweep of k shots is cut (lsrtm_resident.cuh).
 struct PrtmPlan {
   bool ok = false;
-  int slots = 0, cps = 0, rmax = 0, zp = 0, ngroups = 0, ogroups = 0, chunks = 0, cap_rec = 0, cap_ring = 0;
+  int rounds = 0, slots = 0, cps = 0, rmax = 0, zp = 0, ngroups = 0, ogroups = 0, chunks = 0, cap_rec = 0, cap_ring = 0;
+  double march = 0;   // estimated issue time of a step's rows, thousands of cycles
   size_t smem = 0, halo = 0;
 };
 constexpr int kPrtmHelpers = 3;   // warps for records, rings and data beside the march (1 shot, migration: 6.6 / 4.7 / 4.3 us a step with 1 / 2 / 3)
@@ -598,8 +599,9 @@ class Prtm {
     int cps = 1;
     for (need(cps); p.smem > kPrtmMaxSmem && cps < most;) need(++cps);
     if (p.smem > kPrtmMaxSmem) return p;
-    const int fit = std::max(1, sms_ / cps), rounds = (kmax_ + fit - 1) / fit;
-    p.slots = (kmax_ + rounds - 1) / rounds;
+    const int fit = std::max(1, sms_ / cps);
+    p.rounds = (kmax_ + fit - 1) / fit;
+    p.slots = (kmax_ + p.rounds - 1) / p.rounds;
     p.cps = std::min(most, sms_ / p.slots);
     need(p.cps);
     p.halo = (size_t)p.slots * p.cps * (mode == PRTM_SOURCE ? 1 : 2) * 4 * 4 * p.ogroups + 1;   // and the launch's flag
@@ -618,12 +620,37 @@ class Prtm {
       }
     }
     p.ok = p.chunks > 0;
+    p.march = best * 1e-3;
     return p;
+  }
+  // Estimated microseconds a step of a batch, on chip and launched (fits to
+  // 106 operators of 8..3000 x 30..1800 cells and 1..500 shots, within 18 %
+  // and 25 %).  A round of slots costs its barriers, its largest slab's march
+  // and the polling of the edge rows, which grows with the depth: grids of a
+  // thousand cells and more in depth, cut into slabs of two or three rows, are
+  // the launched loops' (46 x 1250, 1 shot: modelling 6.6 on chip against 5.1,
+  // migration 17.0 against 10.4; 36 x 1521, reference arithmetic: 7.9 against
+  // 4.9 a shot), where 20 shots of 521 x 211 take 9.9 against 33.
+  double resident_us(int mode) const {
+    const PrtmPlan &p = plan_[mode];
+    const bool ref = arith_ == ARITH_REF;
+    if (mode == PRTM_BORN)
+      return p.rounds * (ref ? 0.76 + 1.49 * p.march + 0.0121 * p.ogroups : 1.23 + 0.82 * p.march + 0.0120 * p.ogroups);
+    const double part = mode == PRTM_SOURCE ? 0.5 : 1.0;   // one pair of fields
+    return p.rounds * (ref ? 0.89 + part * (1.15 * p.march + 0.0227 * p.ogroups)
+                           : 1.21 + part * (0.72 * p.march + 0.0223 * p.ogroups));
+  }
+  double launched_us(bool adj) const {
+    const double m = 1e-6 * kmax_ * fsz();
+    if (arith_ == ARITH_REF) return adj ? 9.5 + 15.8 * m : 4.3 + 9.2 * m;
+    return adj ? 9.1 + 20.0 * m : 4.05 + 13.5 * m;
   }
   bool resident(bool adj) const {
     if (!use_resident_) return false;
-    if (!adj) return plan_[PRTM_BORN].ok;
-    return plan_[PRTM_SOURCE].ok && plan_[adj_mode_ == SWFWI_PRTM_ADJ_EXACT ? PRTM_TRANSPOSE : PRTM_MIGRATE].ok;
+    const double limit = 0.9 * launched_us(adj);
+    if (!adj) return plan_[PRTM_BORN].ok && resident_us(PRTM_BORN) < limit;
+    const int back = adj_mode_ == SWFWI_PRTM_ADJ_EXACT ? PRTM_TRANSPOSE : PRTM_MIGRATE;
+    return plan_[PRTM_SOURCE].ok && plan_[back].ok && resident_us(PRTM_SOURCE) + resident_us(back) < limit;
   }
   // one sweep over the k shots from s0 (the batch's first), images (or the
   // model of k == 1) in img

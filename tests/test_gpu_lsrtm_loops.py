@@ -133,3 +133,39 @@ def test_thin_sponge_ring_is_saved_whole(cuda, arith, nb):
         np.testing.assert_array_equal(out[1], out[0])
     else:
         assert rel_l2(out[1], out[0]) < 2e-4
+
+
+@pytest.mark.parametrize("arith,nx,nz,ns,nb,on_chip", [
+    (1, 120, 90, 3, 20, True), (0, 120, 90, 2, 20, True), (1, 300, 400, 6, 20, True), (0, 400, 300, 2, 20, True),
+    (1, 46, 1250, 1, 20, False), (0, 36, 1521, 2, 10, False), (1, 70, 1329, 11, 10, False),
+])
+def test_the_faster_form_is_chosen(cuda, arith, nx, nz, ns, nb, on_chip):
+    """Deep grids, which on-chip sweeps cut into slabs of two or three rows,
+    take the launched loops, with their bits; others the sweeps."""
+    import swfwi_b200 as S
+    nt = 60
+    rng = np.random.default_rng(nx)
+    vel = t(cuda, rng.uniform(1500, 2500, (nx, nz)).astype(np.float32))
+    mod = t(cuda, rng.standard_normal((nx, nz)).astype(np.float32))
+    dat = t(cuda, rng.standard_normal((ns, nx, nt)).astype(np.float32))
+    out = []
+    for resident in (True, False):
+        op = S.Prtm2d(vel, dz=10.0, dx=10.0, dt=0.001, amp=1.0, fm=25.0, nb=nb, nt=nt, ns=ns, ng=nx, sxbeg=0, szbeg=1,
+                      jsx=(nx - 1) // ns, jsz=0, gxbeg=0, gzbeg=2, jgx=1, jgz=0, arith=arith)
+        op.set_resident(resident)
+        for exact in (False, True):
+            op.set_adjoint(S.PRTM_ADJ_EXACT if exact else S.PRTM_ADJ_REFERENCE)
+            for adj in (False, True):
+                o = cuda.zeros_like(mod if adj else dat)
+                cuda.cuda.synchronize()
+                S.stats_reset()
+                op.lop(adj, False, o if adj else mod, dat if adj else o)
+                launches = S.stats_read()["kernel_launches"]
+                assert (launches < nt) == (resident and on_chip), (exact, adj, launches)
+                out.append(o.cpu().numpy())
+        op.close()
+    for a, b in zip(out[:4], out[4:]):
+        if on_chip and arith == S.ARITH_FAST:
+            assert rel_l2(a, b) < 2e-4
+        else:
+            np.testing.assert_array_equal(a, b)
