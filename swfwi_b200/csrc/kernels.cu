@@ -379,17 +379,21 @@ static void step_t(const StepArgs &a, int nslots, cudaStream_t st) {
 }
 
 // Tiles of 16 rows and 512 threads while 32-row tiles would be fewer than four
-// an SM: their phases are a quarter of the passes.  Microseconds a launch in
-// a row of them, reference arithmetic, 16 x 512 against 32 x 256: 533 x 193
-// (102 tiles of 32 rows) 4.9 / 6.4, 1000 x 400 (403) 7.2 / 8.4, 1500 x 600
-// (893) 12.7 / 11.4, 3000 x 1000 37 / 29.  (The launch without programmatic
-// serialisation, 32 x 256: 7.2 and 9.5 on the first two.)
-constexpr long long kSmallTiles = 4 * 148;
+// an SM (FAST: six): their phases are a quarter of the passes.  Microseconds a
+// launch in a row of them, 16 x 512 against 32 x 256.  Reference arithmetic:
+// 533 x 193 (102 tiles of 32 rows) 4.9 / 6.4, 1000 x 400 (403) 7.2 / 8.4, 1000
+// x 700 (682) 10.6 / 10.6, 3 fields of 1000 x 250 (744) 11.3 / 10.7, 1500 x
+// 600 (893) 12.7 / 11.4, 3000 x 1000 37 / 29.  FAST: 12 fields of 814 x 72
+// (624) 9.2 / 12.5, 744 tiles 10.6 / 12.3, 880 11.8 / 12.3, 1024 13.4 / 12.5.
+// (32 x 256 without programmatic serialisation: 7.2 and 9.5 on the first two,
+// 11.3 on FAST's 624.)
+template <int ARITH>
+constexpr long long kSmallTiles = (ARITH == ARITH_FAST ? 6 : 4) * 148;
 
 template <int ARITH, bool DAMPED, bool RCP>
 static void step_tx(const StepArgs &a, int nslots, cudaStream_t st) {
   const long long tiles = (long long)((a.nz - 12 + kTZ - 1) / kTZ) * ((a.nx - 12 + 31) / 32) * nslots;
-  if (tiles <= kSmallTiles) step_t<ARITH, DAMPED, RCP, 16, 512>(a, nslots, st);
+  if (tiles <= kSmallTiles<ARITH>) step_t<ARITH, DAMPED, RCP, 16, 512>(a, nslots, st);
   else step_t<ARITH, DAMPED, RCP, 32, 256>(a, nslots, st);
 }
 
