@@ -84,6 +84,23 @@ class Scratch {
   bool idle_ = false;
 };
 
+// A word of host memory that kernels can write, zero at first.  The words of a
+// context share one page, which pinning costs a millisecond or two once.
+// Whoever holds a word ends its work before giving it back.
+class HostWord {
+ public:
+  HostWord();
+  ~HostWord();
+  HostWord(const HostWord &) = delete;
+  HostWord &operator=(const HostWord &) = delete;
+  int *get() const { return p_; }
+  int value() const { return *static_cast<volatile int *>(p_); }
+  void clear() { *static_cast<volatile int *>(p_) = 0; }
+
+ private:
+  int *p_ = nullptr;
+};
+
 // Owning device allocation (cudaMalloc / cudaFree).
 template <typename T>
 class DevBuf {

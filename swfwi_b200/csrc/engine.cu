@@ -279,6 +279,7 @@ void Propagator::set_receivers_per_shot(const int *offsets, const int *gx, const
     m = std::max(m, c);
   }
   ngmax = m;
+  own_receivers_ = true;
   h_rec_count.resize(ns);
   h_rec_x.assign((size_t)ns * ngmax, -1);
   h_rec_z.assign((size_t)ns * ngmax, -1);
@@ -383,7 +384,8 @@ void Propagator::upload_geometry() {
         (sz[i] >= nzpad - bx0 || sx[i] < bx0 || sx[i] >= nxpad - bx0))
       src_in_strips_ = true;
   rec_unused_ = false;
-  for (int s = 0; s < ns; s++) {
+  if (!own_receivers_) row_rec_ = row_geo_;   // the common line
+  for (int s = 0; s < ns && own_receivers_; s++) {
     std::vector<int> h(nxpad, 0);
     for (int i = 0; i < ngmax; i++) {
       const int x = rx[(size_t)s * ngmax + i];

@@ -221,6 +221,7 @@ class Propagator {
   // points per padded row, the most of any slot: one shot's source, all
   // sources, one shot's receivers, the common receiver line
   std::vector<int> row_src1_, row_src_, row_rec_, row_geo_;
+  bool own_receivers_ = false;  // receivers were set per shot
   bool rec_unused_ = false;     // some shots have fewer than ngmax receivers
   bool src_in_strips_ = false;  // some source is a cell of the boundary strips
   DevBuf<uint4> res_halo_;      // edge rows of the resident time loop

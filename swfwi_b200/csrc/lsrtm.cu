@@ -433,7 +433,7 @@ class Prtm {
     const size_t per_shot = sizeof(float) * (5 * fsz + (size_t)nt * 4 * (nx + nz) + (size_t)nx * nz);
     kmax_ = arith == ARITH_REF ? 1 : (int)std::max<size_t>(1, std::min<size_t>(ns, kBatchBudget / per_shot));
     kmax_ = std::min(kmax_, 65535);
-    for (DevBuf<float> *f : {&sp0_, &sp1_, &gp0_, &gp1_, &gp2_}) {
+    for (DevBuf<float> *f : {&sp0_, &sp1_, &gp0_, &gp1_}) {
       f->resize((size_t)kmax_ * fsz);
       f->zero(st);
     }
@@ -449,9 +449,6 @@ class Prtm {
       }
     }
     geo_serial_ = ng > 1 && jgx == 0 && jgz == 0;
-    // written by a sweep that gives up, read by the host without a copy
-    SWFWI_CUDA(cudaHostAlloc(&err_, sizeof(int), cudaHostAllocMapped));
-    *err_ = 0;
     int dev = 0;
     SWFWI_CUDA(cudaGetDevice(&dev));
     SWFWI_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
@@ -460,13 +457,18 @@ class Prtm {
       plan_[m] = plan_resident_sweep(m);
       if (plan_[m].ok) halo = std::max(halo, plan_[m].halo);
     }
-    halo_.resize(halo);
+    // behind the scratch field: an allocation of its own would take a quarter
+    // of a millisecond of the operator's 1.1
+    const size_t field = ((size_t)kmax_ * fsz + 3) / 4 * 4;
+    gp2_.resize(field + 4 * halo);
+    gp2_.zero(st);
+    halo_ = reinterpret_cast<uint4 *>(gp2_.get() + field);
     geo_ = PrtmGeo{nx, nz, nb, nxpad_, nzpad_, nt, ng, (long long)fsz, spos_.get(), rpos_.get(), sponge_.get(),
                    ng > 1 && jgx == 0 && jgz == 0 ? 1 : 0};
   }
 
   ~Prtm() {
-    if (err_) cudaFreeHost(err_);   // waits for the sweeps in flight
+    cudaDeviceSynchronize();   // the sweeps in flight may still raise err_
     for (Graph &g : graphs_)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     if (cap_) cudaStreamDestroy(cap_);
@@ -568,9 +570,9 @@ class Prtm {
 
   // ---- resident sweeps ----
   void report() {
-    if (!*static_cast<volatile int *>(err_)) return;
+    if (!err_.value()) return;
     SWFWI_CUDA(cudaDeviceSynchronize());   // the sweep's other blocks have raised it too
-    *static_cast<volatile int *>(err_) = 0;
+    err_.clear();
     throw Error(SWFWI_ERR_TIMEOUT, "a resident sweep's bounded wait on its neighbours gave up");
   }
   PrtmPlan plan_resident_sweep(int mode) const {
@@ -688,11 +690,11 @@ class Prtm {
       a.ring = ring_.get() + c * a.ring_stride;
       a.img = img ? img + c * img_stride : nullptr;
       a.img_stride = img_stride;
-      a.halo = halo_.get();
+      a.halo = halo_;
       a.quit = reinterpret_cast<int *>(a.halo + p.halo - 1);
-      a.err = err_;
+      a.err = err_.get();
       a.patience = wait_limit_;
-      SWFWI_CUDA(cudaMemsetAsync(halo_.get(), 0, sizeof(uint4) * p.halo, st));
+      SWFWI_CUDA(cudaMemsetAsync(halo_, 0, sizeof(uint4) * p.halo, st));
       if (arith_ == ARITH_REF) prtm_resident_mode<ARITH_REF>(mode, a, p.smem, st);
       else prtm_resident_mode<ARITH_FAST>(mode, a, p.smem, st);
     }
@@ -935,8 +937,8 @@ class Prtm {
   int sms_ = 148;
   PrtmPlan plan_[4];               // by PrtmSweep
   std::vector<int> row_rec_;
-  DevBuf<uint4> halo_;
-  int *err_ = nullptr;             // mapped host memory
+  uint4 *halo_ = nullptr;          // the sweeps' exchange buffer, in gp2_
+  HostWord err_;                   // written by a sweep that gives up, read without a copy
   long long wait_limit_ = 1LL << 31;
   PrtmCoef c_{};
   PrtmGeo geo_{};

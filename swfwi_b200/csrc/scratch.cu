@@ -4,7 +4,8 @@
 // a third of an ensemble analysis of 64 members.  So one buffer per CUDA
 // context, of at most kKeepBytes, is kept between such calls; a second
 // concurrent call allocates its own, and an allocation of this library that
-// finds the device full frees the kept ones before it gives up.
+// finds the device full frees the kept ones before it gives up.  Below it, the
+// page of host words of a context.
 #include <cuda.h>
 #include <mutex>
 #include <vector>
@@ -81,6 +82,72 @@ Scratch::~Scratch() {
     }
   }
   if (drop) cudaFree(drop);
+}
+
+namespace {
+
+constexpr int kPageWords = 1024;   // 4 KB
+struct Page {
+  int dev;
+  unsigned long long ctx;   // 0: a page of its own, freed with its word
+  int *base;
+  std::vector<int> free;    // word numbers not held
+};
+std::vector<Page> g_pages;
+
+int *pinned(size_t words) {
+  void *p = nullptr;
+  SWFWI_CUDA(cudaHostAlloc(&p, words * sizeof(int), cudaHostAllocMapped));
+  return static_cast<int *>(p);
+}
+
+}  // namespace
+
+HostWord::HostWord() {
+  int dev = 0;
+  SWFWI_CUDA(cudaGetDevice(&dev));
+  const unsigned long long ctx = context_id();
+  std::lock_guard<std::mutex> g(g_mu);
+  Page *page = nullptr;
+  for (Page &q : g_pages)
+    if (ctx && q.ctx == ctx && !q.free.empty()) page = &q;
+  if (!page) {
+    // pages that nobody holds a word of, of contexts this device had before,
+    // are gone with those
+    for (size_t i = g_pages.size(); i-- > 0;)
+      if (g_pages[i].dev == dev && g_pages[i].ctx != ctx && (int)g_pages[i].free.size() == kPageWords)
+        g_pages.erase(g_pages.begin() + i);
+    Page q{dev, ctx, pinned(ctx ? kPageWords : 1), {}};
+    for (int i = (ctx ? kPageWords : 1) - 1; i >= 0; i--) q.free.push_back(i);
+    g_pages.push_back(std::move(q));
+    page = &g_pages.back();
+  }
+  p_ = page->base + page->free.back();
+  page->free.pop_back();
+  *p_ = 0;
+}
+
+HostWord::~HostWord() {
+  std::lock_guard<std::mutex> g(g_mu);
+  for (size_t i = 0; i < g_pages.size(); i++) {
+    Page &q = g_pages[i];
+    if (p_ < q.base || p_ >= q.base + (q.ctx ? kPageWords : 1)) continue;
+    if (!q.ctx) {
+      cudaFreeHost(q.base);
+      g_pages.erase(g_pages.begin() + i);
+      return;
+    }
+    q.free.push_back((int)(p_ - q.base));   // room for it was there before
+    // one page a context stays; others go when their last word does
+    if ((int)q.free.size() == kPageWords)
+      for (size_t j = 0; j < g_pages.size(); j++)
+        if (j != i && g_pages[j].ctx == q.ctx) {
+          cudaFreeHost(q.base);
+          g_pages.erase(g_pages.begin() + i);
+          break;
+        }
+    return;
+  }
 }
 
 void *device_alloc(size_t bytes) {

@@ -110,3 +110,33 @@ def test_lsrtm(cuda, arith, adj, exact):
     assert torch.equal(run(op), want)
     op.check()
     op.close()
+
+
+def test_operators_report_for_themselves(cuda):
+    """Several operators alive, made and closed in turn: one that gave up is
+    the only one to say so, and a new one starts clean."""
+    import swfwi_b200 as S
+    torch = cuda
+    nx, nz, nt, ng = 200, 60, 100, 100
+    vel = torch.full((nx, nz), 2000.0, device="cuda")
+    mod = torch.ones((nx, nz), device="cuda")
+    dat = torch.zeros((1, ng, nt), device="cuda")
+
+    def make():
+        return S.Prtm2d(vel, dz=10.0, dx=10.0, dt=0.001, amp=1.0, fm=25.0, nb=20, nt=nt, ns=1, ng=ng, sxbeg=50, szbeg=2,
+                        jsx=0, jsz=0, gxbeg=0, gzbeg=2, jgx=1, jgz=0, arith=S.ARITH_FAST)
+
+    ops = [make() for _ in range(5)]
+    ops[2].set_wait_limit(0)
+    for op in ops:
+        op.lop(False, False, mod, dat)
+    torch.cuda.synchronize()
+    for k in (0, 1, 3, 4):
+        ops[k].check()
+    ops[2].close()                              # unasked
+    fresh = make()                              # may take over its word
+    fresh.lop(False, False, mod, dat)
+    fresh.check()
+    for op in (*ops[:2], *ops[3:], fresh):
+        op.check()
+        op.close()
