@@ -104,6 +104,7 @@ class Damp4t10d {
   void FwiForwardModeling(const std::vector<float> &encsrc, std::vector<float> &dcal, int shot_id) const {
     swfwi_cpp::DeviceFloats w(encsrc.data(), (size_t)nt_), d((size_t)nt_ * getng());
     swfwi_cpp::check(swfwi_damp4t10d_fwi_forward_modeling(h_, w.ptr(), d.ptr(), shot_id));
+    swfwi_cpp::check(swfwi_damp4t10d_check(h_));
     dcal.resize((size_t)nt_ * getng());
     d.get(dcal.data());
   }
@@ -113,6 +114,7 @@ class Damp4t10d {
   void EssForwardModeling(const std::vector<float> &encsrc, std::vector<float> &dcal) const {
     swfwi_cpp::DeviceFloats w(encsrc.data(), (size_t)nt_ * getns()), d((size_t)nt_ * getng());
     swfwi_cpp::check(swfwi_damp4t10d_ess_forward_modeling(h_, w.ptr(), d.ptr()));
+    swfwi_cpp::check(swfwi_damp4t10d_check(h_));
     dcal.resize((size_t)nt_ * getng());
     d.get(dcal.data());
   }

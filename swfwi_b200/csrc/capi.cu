@@ -491,6 +491,7 @@ int swfwi_gradient_host(swfwi_damp4t10d *h, const float *exvel, const float *wlt
     SWFWI_CUDA(cudaStreamSynchronize(st));
     if (old) p.bind_velocity(old);
     else p.unbind_velocity(h->hv.get());
+    if (!obj) p.check_device_error();   // with objectives the batch has done so
   });
 }
 

@@ -140,3 +140,24 @@ def test_operators_report_for_themselves(cuda):
     for op in (*ops[:2], *ops[3:], fresh):
         op.check()
         op.close()
+
+
+def test_host_gradient_without_objectives_reports(cuda):
+    import ctypes as C
+    import swfwi_b200 as S
+    torch = cuda
+    s, m, vel, wlt = propagator(torch, S.ARITH_FAST)
+    v, w = vel.cpu().numpy(), wlt.cpu().numpy()
+    d, g, ids = np.zeros((3, s.nt, s.ng), np.float32), np.zeros_like(v), np.arange(3, dtype=np.int32)
+
+    def call():
+        f, i = C.POINTER(C.c_float), C.POINTER(C.c_int)
+        S._check(S.lib().swfwi_gradient_host(m.h, v.ctypes.data_as(f), w.ctypes.data_as(f), d.ctypes.data_as(f),
+                                             ids.ctypes.data_as(i), 3, g.ctypes.data_as(f), None))
+
+    call()
+    m.set_wait_limit(0)
+    raises_timeout(call)
+    m.set_wait_limit(LIMIT)
+    call()
+    m.check()
