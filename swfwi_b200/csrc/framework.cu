@@ -272,7 +272,7 @@ void FwiRunner::regu_epoch(int iter) {
                    p_.dx, search.maxdv, st);
   float a2max = 0;
   SWFWI_CUDA(cudaMemcpyAsync(&a2max, scratch_.get(), sizeof(float), cudaMemcpyDeviceToHost, st));
-  SWFWI_CUDA(cudaStreamSynchronize(st));
+  p_.check_device_error();   // waits; a sweep that gave up ends the epoch
   float a3max = 2 * a2max;
   auto f = [&](float alpha) -> float {
     launch_update_vel(trial_.get(), vel_.get(), dir_.get(), n_, alpha, vmin_t_, vmax_t_, st);
@@ -284,6 +284,7 @@ void FwiRunner::regu_epoch(int iter) {
   };
   float objv = 0;
   float step = search.calsteplen(f, obj1, a3max, objv);
+  p_.check_device_error();   // before the model changes
   update_obj = objv;
   launch_update_vel(vel_.get(), vel_.get(), dir_.get(), n_, step, vmin_t_, vmax_t_, st);
   launch_refill_boundary(vel_.get(), p_.nxpad, p_.nzpad, p_.bz0, p_.bzn, p_.bx0, p_.bxn, st);
@@ -413,6 +414,7 @@ void FwiRunner::ess_epoch(int iter) {
   launch_trans_vsrc(vsrc_.get(), res_.get(), nt, ng, 1, st);
   g_.zero(st);
   p_.calgradient_ess(encsrc_.get(), vsrc_.get(), g_.get());
+  p_.check_device_error();   // before the gradient enters the search direction's history
   p_.scale_gradient(g_.get());
   p_.mask_gradient(g_.get());
   update_grad(iter);
@@ -433,6 +435,7 @@ void FwiRunner::ess_epoch(int iter) {
   };
   float objv = 0;
   float step = search.calsteplen(f, obj1, a3max, objv);
+  p_.check_device_error();   // before the model changes
   update_obj = objv;
   launch_update_vel(vel_.get(), vel_.get(), dir_.get(), n_, step, vmin_t_, vmax_t_, st);
   launch_refill_boundary(vel_.get(), p_.nxpad, p_.nzpad, p_.bz0, p_.bzn, p_.bx0, p_.bxn, st);

@@ -161,3 +161,22 @@ def test_host_gradient_without_objectives_reports(cuda):
     m.set_wait_limit(LIMIT)
     call()
     m.check()
+
+
+@pytest.mark.parametrize("regularised", [False, True])
+def test_encoded_epoch_reports_and_keeps_its_model(cuda, regularised):
+    import swfwi_b200 as S
+    torch = cuda
+    s, m, vel, wlt = propagator(torch, S.ARITH_FAST)
+    dobs = np.random.default_rng(1).standard_normal((3, s.nt, s.ng)).astype(np.float32)
+    fw = S.EssFwiFramework(m, vel.cpu().numpy(), s.vmin, s.vmax, s.nita, s.maxdv, wlt.cpu().numpy(), dobs)
+    if regularised:
+        fw.setRegularization(1.0, 1.0)
+    fw.epoch(0)
+    before = fw.velocity()
+    m.set_wait_limit(0)
+    raises_timeout(lambda: fw.epoch(1))
+    np.testing.assert_array_equal(fw.velocity(), before)
+    m.set_wait_limit(LIMIT)
+    fw.epoch(1)
+    assert np.isfinite(fw.velocity()).all() and not np.array_equal(fw.velocity(), before)
