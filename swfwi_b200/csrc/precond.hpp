@@ -20,7 +20,8 @@
 // every product accumulates in FP32 on the tensor cores (tcgen05.mma
 // kind::f16, BF16 operands, accumulators in tensor memory); master weights,
 // Adam moments, gradients, the loss and the output layer are FP32.  H and W
-// must be multiples of 8; every width a multiple of 16, at most 128.
+// must be multiples of 8; every width a multiple of 16, at most 64 (a
+// concatenation's then at most 128).
 #pragma once
 #include <cuda_bf16.h>
 #include <cstdint>
