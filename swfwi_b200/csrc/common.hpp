@@ -99,6 +99,7 @@ class HostWord {
 
  private:
   int *p_ = nullptr;
+  unsigned long long ctx_ = 0;   // context of its page
 };
 
 // Owning device allocation (cudaMalloc / cudaFree).

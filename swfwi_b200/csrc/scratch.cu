@@ -106,17 +106,16 @@ int *pinned(size_t words) {
 HostWord::HostWord() {
   int dev = 0;
   SWFWI_CUDA(cudaGetDevice(&dev));
-  const unsigned long long ctx = context_id();
+  const unsigned long long ctx = ctx_ = context_id();
   std::lock_guard<std::mutex> g(g_mu);
   Page *page = nullptr;
   for (Page &q : g_pages)
     if (ctx && q.ctx == ctx && !q.free.empty()) page = &q;
   if (!page) {
-    // pages that nobody holds a word of, of contexts this device had before,
-    // are gone with those
-    for (size_t i = g_pages.size(); i-- > 0;)
-      if (g_pages[i].dev == dev && g_pages[i].ctx != ctx && (int)g_pages[i].free.size() == kPageWords)
-        g_pages.erase(g_pages.begin() + i);
+    // pages of contexts this device had before are gone with those; a word
+    // held beyond them finds no page any more
+    for (size_t i = g_pages.size(); ctx && i-- > 0;)
+      if (g_pages[i].dev == dev && g_pages[i].ctx && g_pages[i].ctx != ctx) g_pages.erase(g_pages.begin() + i);
     Page q{dev, ctx, pinned(ctx ? kPageWords : 1), {}};
     for (int i = (ctx ? kPageWords : 1) - 1; i >= 0; i--) q.free.push_back(i);
     g_pages.push_back(std::move(q));
@@ -131,7 +130,7 @@ HostWord::~HostWord() {
   std::lock_guard<std::mutex> g(g_mu);
   for (size_t i = 0; i < g_pages.size(); i++) {
     Page &q = g_pages[i];
-    if (p_ < q.base || p_ >= q.base + (q.ctx ? kPageWords : 1)) continue;
+    if (q.ctx != ctx_ || p_ < q.base || p_ >= q.base + (q.ctx ? kPageWords : 1)) continue;
     if (!q.ctx) {
       cudaFreeHost(q.base);
       g_pages.erase(g_pages.begin() + i);
